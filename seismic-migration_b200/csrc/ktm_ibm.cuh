@@ -27,7 +27,8 @@ __device__ __forceinline__ float pow2_exact(int e)
     return 0.0f;
 }
 
-__device__ __forceinline__ float ibm32_to_f32(uint32_t w)
+// every word, the infinite powers and the 0 * inf case among them
+static __device__ __noinline__ float ibm32_any(uint32_t w)
 {
     const float sign = (w & 0x80000000u) ? -1.0f : 1.0f;
     const float q = __fdiv_rn(__uint2float_rn(w & 0x00ffffffu), 16777215.0f);
@@ -37,6 +38,29 @@ __device__ __forceinline__ float ibm32_to_f32(uint32_t w)
     // is what the reference writes; the device's canonical NaN differs in bits.
     if (q == 0.0f && e * 4 > 127) return __int_as_float(0xffc00000);
     return __fmul_rn(__fmul_rn(sign, q), p);
+}
+
+// Words whose power of two is a normal number (exponents 33 to 95), and zeros with smaller
+// ones: one multiply for the quotient, one residual step (for all 2^24 fractions it gives
+// the correctly rounded quotient) and the power from its bits, about 12 instructions and no
+// branch.  Sets `other` for a word that ibm32_any has to convert.  All 2^32 words give the
+// same bits by the two together as by ibm32_any alone (checked on the GPU).  4097 traces of
+// 1001 words through the 2.5D filter: 17 us, with the division and its selects per word 29.
+__device__ __forceinline__ float ibm32_usual(uint32_t w, bool& other)
+{
+    const uint32_t e = w & 0x7f000000u, m = w & 0x00ffffffu;
+    other = other || e > 0x5f000000u || (e < 0x21000000u && m != 0u);
+    const float f = __uint2float_rn(m), r = 1.0f / 16777215.0f;
+    const float q0 = __fmul_rn(f, r);
+    const float q = __fmaf_rn(__fmaf_rn(-16777215.0f, q0, f), r, q0);
+    // 2^(4 (E - 64)) with the word's sign: (4 E - 256 + 127) << 23
+    return __fmul_rn(q, __uint_as_float(((max(e, 0x21000000u) << 1) - (129u << 23)) | (w & 0x80000000u)));
+}
+__device__ __forceinline__ float ibm32_to_f32(uint32_t w)
+{
+    bool other = false;
+    const float v = ibm32_usual(w, other);
+    return other ? ibm32_any(w) : v;
 }
 
 }  // namespace dev
