@@ -30,18 +30,28 @@
 //            traces (blockIdx.z); slices write partial images that a second
 //            kernel sums in a fixed order (deterministic), so small images still
 //            fill the GPU;
-//   traces stream through shared memory in chunks, double-buffered: thread 0
-//   moves a chunk's packed rows (one contiguous, 16-byte aligned range) with a
-//   single bulk copy (cp.async.bulk) completed on the buffer's mbarrier, waited
-//   for with a one-second bound; the coordinates and scales follow in 4-byte
-//   cp.async.  For each chunk, lane c of every warp computes trace c's squared
-//   distances and skip flag (aperture, or a lower bound of u over the run beyond
-//   the trace end) for the warp's column; the warp walks the kept traces of its
-//   ballot, taking their distances by shuffle, with no second barrier per chunk.
+//   traces stream through shared memory in chunks of up to 32, in two or three
+//   buffers: one thread moves a chunk's packed rows (one contiguous, 16-byte
+//   aligned range) with a single bulk copy (cp.async.bulk) completed on the
+//   buffer's mbarrier, which every warp waits on with a one-second bound.  No
+//   barrier of the CTA: a warp goes on to the next chunk as soon as it is through
+//   with one, and the last warp through refills the buffer.  For each chunk, lane c
+//   of every warp reads trace c's coordinates and computes its squared distances,
+//   scale and reach (aperture, or a lower bound of u beyond the trace end) for the
+//   warp's column; the kept traces go in order into a table of the warp in shared
+//   memory, one 16-byte entry each, which the warp then walks.
 //   ktmAutotuneTile picks R, the shape and the chunk per job.
+// What bounds it: two special-function square roots a pair take 16 cycles of a
+// scheduler; the pair loop alone runs at 19 (24 warps, 13 instructions a pair), the
+// kernel at 21 to 22 with the chunks' geometry (about 1800 cycles of an SM per chunk),
+// the table walk and the CTA's prologue and end.  Against two CTA barriers' worth of
+// waiting per chunk, shuffles and a bit search per trace: 200 x 200 x 1501 image, 2500
+// FP16 traces 52.7 ms instead of 56.6; 256 x 1001, 16,384 FP16 traces 2.27 ms instead of
+// 2.34; 128 x 751, 6144 FP32 traces with the table weight 0.46 ms instead of 0.52.
 #include "ktm_pair.cuh"
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 namespace ktm {
@@ -52,8 +62,8 @@ namespace {
 // registers capped at 80 (65,536 / 768 threads); MB x (budget + up to 1 KB of
 // static shared memory + the 1 KB the SM reserves) fits the SM's 228 KB.  More
 // columns per CTA share each staged chunk of traces among more warps: on the
-// 200 x 200 x 1501 image, 8192 FP16 traces, 24 x 1 takes 201.8 ms, 12 x 2 203.7
-// ms and 8 x 3 208.6 ms per launch (8 x 2 225.7, 16 x 1 226.8, 4 x 6 229.6).
+// 200 x 200 x 1501 image, 2500 FP16 traces, 24 x 1 takes 52.7 ms, 12 x 2 54.4 and
+// 8 x 3 56.5 per launch.
 // Full = 1: every pick / weight / gradient path is built for the shape; 0: the
 // linear pick with the prefolded or table weight only (the paths the tile
 // tuner searches).
@@ -76,10 +86,7 @@ constexpr bool shape_fits()
 static_assert(shape_fits<Shape24>() && shape_fits<Shape12>() && shape_fits<Shape8>(),
               "each shape's CTAs must fit the SM's 228 KB of shared memory");
 constexpr int kMaxChunk = 32;        // lane c of a warp evaluates trace c of a chunk
-// index of the lowest set bit of a word from its isolated bit times the de Bruijn
-// sequence 0x077CB531 (Leiserson, Prokop and Randall, 1998)
-__constant__ unsigned char kLowBit[32] = {0, 1, 28, 2, 29, 14, 24, 3, 30, 22, 20, 15, 25, 17, 4, 8,
-                                          31, 27, 13, 23, 21, 19, 16, 7, 26, 12, 18, 6, 11, 5, 10, 9};
+constexpr int kMaxStages = 3;
 using namespace dev;
 
 // Bound of one wait for a chunk's bulk copy.  A copy of a chunk takes
@@ -88,28 +95,37 @@ using namespace dev;
 constexpr unsigned long long kBulkWaitNs = 1000000000ull;
 __device__ unsigned g_waitStalls;
 
-// Per-CTA state of the chunk pipeline: one mbarrier per trace-row buffer.
+// Per-CTA state of the chunk pipeline, per row buffer: the mbarrier its copies complete
+// on, how many warps are through with its chunk, how many copies it was given.
 struct ChunkSync {
-    unsigned long long bar[2];
+    unsigned long long bar[kMaxStages];
+    int done[kMaxStages], issued[kMaxStages];
     int stalled;
 };
 static_assert(sizeof(ChunkSync) + sizeof(FastArgs) + sizeof(int) <= 1024,
               "static shared memory of the fast kernels within the 1 KB allowance");
 
+// Traces per row buffer and row buffers of a launch.
+struct Stages {
+    int chunk, stages;
+};
+
 struct ChunkSmem {
-    // layout of one CTA's dynamic shared memory
-    size_t rawBytes, crdOff, wtabOff, total;
+    // layout of one CTA's dynamic shared memory: row buffers, per warp the kept traces'
+    // table and the bounds of the run's steps, the weight table
+    size_t rawBytes, tabOff, stepOff, wtabOff, total;
 };
 
 // table: the kernel interpolates sqrt(j dt) from a per-CTA table (the table weight);
 // the prefolded and sqrt.approx weights need none, and their chunks grow by its size
-__host__ __device__ __forceinline__ ChunkSmem chunk_layout(int chunk, int pitch, int esize, int nt,
+__host__ __device__ __forceinline__ ChunkSmem chunk_layout(Stages st, int warps, int pitch, int esize, int nt,
                                                            bool table)
 {
     ChunkSmem L;
-    L.rawBytes = (size_t)chunk * pitch * esize;              // one buffer
-    L.crdOff = 2 * L.rawBytes;                               // [2][5][chunk] floats
-    L.wtabOff = L.crdOff + ((2 * 5 * (size_t)chunk * 4 + 15) / 16) * 16;
+    L.rawBytes = (size_t)st.chunk * pitch * esize;           // one buffer
+    L.tabOff = st.stages * L.rawBytes;                       // [warps][chunk] float4
+    L.stepOff = L.tabOff + (size_t)warps * st.chunk * 16;    // [warps][8] float2
+    L.wtabOff = L.stepOff + (size_t)warps * 64;
     L.total = L.wtabOff + (table ? (size_t)(nt + 1) * sizeof(float2) : 0);   // [nt+1] weight table
     return L;
 }
@@ -133,55 +149,73 @@ enum { kOutImage = 0, kOutPartial = 1, kOutAtomic = 2 };
 // run runIdx x traces [kb, ke), W = SH::kWarps.  Used by the grid launch (one tile
 // per CTA) and by the persistent batched launch (a queue of tiles from many jobs).
 template <class SH, int R, int PICK, int FMT, int PRE, int GRAD>
-__device__ __forceinline__ bool fast_tile(const FastArgs& a, int chunk, int colGroup, int runIdx,
+__device__ __forceinline__ bool fast_tile(const FastArgs& a, Stages st, int colGroup, int runIdx,
                                           int kb, int ke, float* __restrict__ partial, int outMode,
                                           unsigned char* smem_raw, ChunkSync& cs)
 {
     static_assert(R % 2 == 0, "R pairs");
     using T = typename Elem<FMT>::T;
     const Geometry& g = a.g;
-    const ChunkSmem L = chunk_layout(chunk, a.pitch, sizeof(T), a.g.nt, PRE == kWtTable);
-    T* rawBase = reinterpret_cast<T*>(smem_raw);
-    float* crdBase = reinterpret_cast<float*>(smem_raw + L.crdOff);
+    const int chunk = st.chunk;
+    const ChunkSmem L = chunk_layout(st, SH::kWarps, a.pitch, sizeof(T), a.g.nt, PRE == kWtTable);
     float2* wtab = reinterpret_cast<float2*>(smem_raw + L.wtabOff);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ncols = g.nx * g.ny;
-    const int col = colGroup * SH::kWarps + warp;
-    const bool colValid = col < ncols;
-    const int ci = colValid ? col / g.ny : 0, cj = colValid ? col % g.ny : 0;
+    const int col0 = colGroup * SH::kWarps, active = min(SH::kWarps, ncols - col0);   // warps with a column
+    const bool colValid = warp < active;
+    const int col = colValid ? col0 + warp : 0;
+    const int ci = col / g.ny, cj = col % g.ny;
     const int run0 = runIdx * (32 * R);
     const float invdt = 1.0f / g.dt;
 
     // ---- per-thread tau tables, two tau samples per packed register pair ----
     f2 T2[R / 2], S2[R / 2], acc[R / 2];
-    float t2min = 3.0e38f, smin = 3.0e38f;
+    // Traces that end within the run are walked step by step (200 x 200 x 1501 image, 2500
+    // traces: 52.3 ms against 54.7 without); the other weights and the gradient, whose second
+    // copy of the loop costs more registers than it saves pairs (table weight on a 128 x 751
+    // line: 541 us against 496), evaluate the run to its end, where the guards are zero.
+    constexpr bool kStepwise = PRE == kWtPrefold && GRAD == 0;
+    constexpr int H = R / 2;            // steps of 64 tau samples, one packed pair per lane each
+    // lower bounds of T2' and S' over the run's steps h, h + 1, .. (valid samples)
+    float2* steps = reinterpret_cast<float2*>(smem_raw + L.stepOff) + warp * 8;
+    float2 step[H];
     int nvalid = 0;
 #pragma unroll
     for (int h = 0; h < R / 2; h++) {
         float tv[2], sv[2];
+        step[h] = make_float2(3.0e38f, 3.0e38f);
 #pragma unroll
         for (int e = 0; e < 2; e++) {
             const int l = run0 + lane + 32 * (2 * h + e);
             const bool ok = l < g.nz;
             const int lc = ok ? l : g.nz - 1;
             const float tq = (g.z0 + (float)lc * g.dz) * invdt;
-            const float v = a.velCube ? a.vel[(size_t)(colValid ? col : 0) * g.nz + lc] : a.vel[lc];
+            const float v = a.velCube ? a.vel[(size_t)col * g.nz + lc] : a.vel[lc];
             const float vd = v * g.dt;
             tv[e] = tq * tq;
             sv[e] = 1.0f / (vd * vd);
-            if (ok) { t2min = fminf(t2min, tv[e]); smin = fminf(smin, sv[e]); nvalid++; }
+            if (ok) {
+                step[h] = make_float2(fminf(step[h].x, tv[e]), fminf(step[h].y, sv[e]));
+                nvalid++;
+            }
         }
         T2[h] = pk(tv[0], tv[1]);
         S2[h] = pk(sv[0], sv[1]);
         acc[h] = pk(0.0f, 0.0f);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        t2min = fminf(t2min, __shfl_xor_sync(0xffffffffu, t2min, o));
-        smin = fminf(smin, __shfl_xor_sync(0xffffffffu, smin, o));
-        nvalid += __shfl_xor_sync(0xffffffffu, nvalid, o);
+    for (int h = H - 1; h >= 0; h--) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            step[h].x = fminf(step[h].x, __shfl_xor_sync(0xffffffffu, step[h].x, o));
+            step[h].y = fminf(step[h].y, __shfl_xor_sync(0xffffffffu, step[h].y, o));
+        }
+        if (h + 1 < H) step[h] = make_float2(fminf(step[h].x, step[h + 1].x), fminf(step[h].y, step[h + 1].y));
+        if (lane == 0) steps[h] = step[h];
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) nvalid += __shfl_xor_sync(0xffffffffu, nvalid, o);
     const float colX = g.x0 + (float)ci * g.dx, colY = g.y0 + (float)cj * g.dy;
     if (PRE == kWtTable) {
         for (int j = threadIdx.x; j <= g.nt; j += SH::kThreads) {
@@ -193,164 +227,195 @@ __device__ __forceinline__ bool fast_tile(const FastArgs& a, int chunk, int colG
     const int nchunks = ke > kb ? (ke - kb + chunk - 1) / chunk : 0;
     const size_t rowBytes = (size_t)a.pitch * sizeof(T);
 
-    auto issue = [&](int ch) {
+    // one thread starts chunk ch's copy into its buffer
+    auto issue = [&](int ch, int b) {
         const int k0 = kb + ch * chunk, n = min(chunk, ke - k0);
-        const int b = ch & 1;
-        unsigned char* dst = reinterpret_cast<unsigned char*>(rawBase) + b * L.rawBytes;
-        const unsigned char* src = static_cast<const unsigned char*>(a.traces) + (size_t)k0 * rowBytes;
-        if (threadIdx.x == 0) bulk_g2s(dst, src, (unsigned)((size_t)n * rowBytes), &cs.bar[b]);
-        float* crd = crdBase + b * 5 * chunk;
-        for (int q = threadIdx.x; q < 5 * n; q += SH::kThreads) {
-            const int arr = q / n, c = q % n;
-            const float* srcArr = arr == 0 ? a.midX : arr == 1 ? a.midY : arr == 2 ? a.offX
-                                : arr == 3 ? a.offY : a.scale;
-            cp_async4(crd + arr * chunk + c, srcArr + k0 + c);
-        }
-        cp_async_commit();
+        cs.issued[b]++;
+        bulk_g2s(smem_raw + b * L.rawBytes, static_cast<const unsigned char*>(a.traces) + (size_t)k0 * rowBytes,
+                 (unsigned)((size_t)n * rowBytes), &cs.bar[b]);
     };
 
     const float umax = (float)g.nt;
+    // a first sample past this has no contribution; the margin covers the bounds'
+    // approximate square roots
+    const float upast2 = (umax * 1.0001f + 1.0f) * (umax * 1.0001f + 1.0f);
     const float ap2 = a.aperture > 0.0f ? a.aperture * a.aperture : -1.0f;
     const f2 M2 = pk(kMagic, kMagic);
     unsigned keptTraces = 0;        // traces this warp evaluated (all lanes agree)
 
-    // thread 0 owns both barriers: it arms them, waits on them and invalidates them
     if (threadIdx.x == 0) {
-        mbar_init(&cs.bar[0], 1);
-        mbar_init(&cs.bar[1], 1);
-        cs.stalled = 0;
-    }
-    if (nchunks > 0) issue(0);
-    for (int ch = 0; ch < nchunks; ch++) {
-        const int b = ch & 1;
-        const int k0 = kb + ch * chunk, n = min(chunk, ke - k0);
-        cp_async_wait_all();
-        // the ch/2-th use of buffer b completes phase ch/2 of its barrier
-        if (threadIdx.x == 0 && !mbar_wait_bounded(&cs.bar[b], (ch >> 1) & 1, kBulkWaitNs)) {
-            cs.stalled = 1;
-            atomicAdd(&g_waitStalls, 1u);
-            mbar_wait_bounded(&cs.bar[b], (ch >> 1) & 1, kBulkWaitNs);   // the copy in flight
+        for (int b = 0; b < st.stages; b++) {
+            mbar_init(&cs.bar[b], 1);
+            cs.done[b] = cs.issued[b] = 0;
         }
-        __syncthreads();                       // chunk ch landed; chunk ch-1 fully consumed
-        if (cs.stalled) return false;          // CTA-uniform: no output from this tile
-        if (ch + 1 < nchunks) issue(ch + 1);
-        if (colValid) {
-            // ---- lane c: trace c's distances, scale and skip flag for this column ----
-            // (chunk <= 32); the warp then walks the kept traces in increasing c,
-            // taking their values by shuffle: no shared table, no second barrier
-            const float* crd = crdBase + b * 5 * chunk;
-            float lds_ = 0.0f, ldr_ = 0.0f, lsc = 0.0f;
-            bool keep = false;
-            if (lane < n) {
-                const float mx = crd[lane], my = crd[chunk + lane], ox = crd[2 * chunk + lane],
-                            oy = crd[3 * chunk + lane];
-                lsc = crd[4 * chunk + lane];
-                const float dmx = mx - colX, dmy = my - colY;
-                const float sx = dmx - ox, sy = dmy - oy, rx = dmx + ox, ry = dmy + oy;
-                lds_ = fmaf(sx, sx, sy * sy);           // explicit fusions: the same
-                ldr_ = fmaf(rx, rx, ry * ry);           // values in every build
-                keep = !(ap2 >= 0.0f && fmaf(dmx, dmx, dmy * dmy) > ap2);
-                if (keep) {
-                    // lower bound of u over the run: past the last sample -> no contribution
-                    // approximate square roots: the margin below covers their error
-                    const float ulb = sqrt_approx(fmaf(lds_, smin, t2min)) +
-                                      sqrt_approx(fmaf(ldr_, smin, t2min));
-                    keep = ulb < umax * 1.0001f + 1.0f;
-                }
-            }
-            const unsigned rowsS = smem_u32(reinterpret_cast<const unsigned char*>(rawBase) + b * L.rawBytes);
-            // bits(fl) = kMagicBits + i0: fold the magic offset into the bases (mod 2^32)
-            const unsigned magicT = (unsigned)kMagicBits * (unsigned)sizeof(T);
-            const unsigned wS = smem_u32(wtab) - (unsigned)kMagicBits * 8u;
-            for (unsigned kept = __ballot_sync(0xffffffffu, keep); kept; kept &= kept - 1u) {
-                // lowest kept trace: __ffs at 16 samples a lane, a de Bruijn lookup
-                // (integer multiply, shift, constant table) for shorter runs; 8192 traces,
-                // 512 / 384 / 256-sample runs: 201.3 / 211.5 / 221.3 ms with __ffs,
-                // 202.1 / 202.6 / 218.5 with the lookup
-                const int c = R == 16 ? __ffs(kept) - 1
-                                      : (int)kLowBit[((kept & (0u - kept)) * 0x077CB531u) >> 27];
-                const float ds = __shfl_sync(0xffffffffu, lds_, c);
-                const float dr = __shfl_sync(0xffffffffu, ldr_, c);
-                const float sc = __shfl_sync(0xffffffffu, lsc, c);
-                keptTraces++;
-                const unsigned rowS = rowsS + (unsigned)(c * a.pitch) * (unsigned)sizeof(T) - magicT;
-                const f2 DS = pk(ds, ds), DR = pk(dr, dr), SC = pk(sc, sc);
+        cs.stalled = 0;
+        for (int b = 0; b < st.stages && b < nchunks; b++) issue(b, b);
+    }
+    __syncthreads();                           // barriers, steps and the weight table are ready
+    // Every warp goes through the chunks at its own pace, up to stages - 1 chunks ahead of
+    // the slowest; the last warp through with a chunk refills its buffer.
+    float4* tab = reinterpret_cast<float4*>(smem_raw + L.tabOff) + warp * chunk;
+    for (int ch = 0, b = 0, parity = 0; colValid && ch < nchunks; ch++) {
+        const int k0 = kb + ch * chunk, n = min(chunk, ke - k0);
+        // ---- lane c: trace c's distances, scale, and how many steps of the run it
+        // reaches for this column; the kept traces go in order into the warp's table ----
+        float ds = 0.0f, dr = 0.0f, sc = 0.0f;
+        int hmax = 0;
+        if (lane < n) {
+            const float mx = a.midX[k0 + lane], my = a.midY[k0 + lane], ox = a.offX[k0 + lane],
+                        oy = a.offY[k0 + lane];
+            sc = a.scale[k0 + lane];
+            const float dmx = mx - colX, dmy = my - colY;
+            const float sx = dmx - ox, sy = dmy - oy, rx = dmx + ox, ry = dmy + oy;
+            ds = fmaf(sx, sx, sy * sy);             // explicit fusions: the same
+            dr = fmaf(rx, rx, ry * ry);             // values in every build
+            // lower bound of u from step h on: steps past the last sample contribute zero
+            auto reaches = [&](int h) {
+                const float2 m = steps[h];      // (sqrt(as) + sqrt(ar))^2 = as + ar + 2 sqrt(as ar)
+                const float as = fmaf(ds, m.y, m.x), ar = fmaf(dr, m.y, m.x);
+                return fmaf(2.0f, sqrt_approx(as * ar), as + ar) < upast2;
+            };
+            if (!(ap2 >= 0.0f && fmaf(dmx, dmx, dmy * dmy) > ap2) && reaches(0)) {
+                hmax = 1;
 #pragma unroll
-                for (int h = 0; h < R / 2; h++) {
-                    if (GRAD) {
-                        // d/dS' of |tau| s_k W(u) V(u), u = sqrt(a_s) + sqrt(a_r):
-                        // (dW/du V + W dV/du) du/dS', du/dS' = Ds/(2 sqrt a_s) + Dr/(2 sqrt a_r)
-                        float as0, as1, ar0, ar1;
-                        upk(fma2(DS, S2[h], T2[h]), as0, as1);
-                        upk(fma2(DR, S2[h], T2[h]), ar0, ar1);
-                        const f2 RS = pk(fminf(rsqrt_approx(as0), 3.0e38f), fminf(rsqrt_approx(as1), 3.0e38f));
-                        const f2 RR = pk(fminf(rsqrt_approx(ar0), 3.0e38f), fminf(rsqrt_approx(ar1), 3.0e38f));
-                        f2 U = fma2(pk(ar0, ar1), RR, mul2(pk(as0, as1), RS));
-                        float u0, u1;
-                        upk(U, u0, u1);
-                        u0 = fminf(u0, umax);
-                        u1 = fminf(u1, umax);
-                        U = pk(u0, u1);
-                        const f2 FL = add2_rm(U, M2);
-                        float fl0, fl1;
-                        upk(FL, fl0, fl1);
-                        const unsigned q0 = __float_as_uint(fl0), q1 = __float_as_uint(fl1);
-                        const f2 F = sub2(U, sub2(FL, M2));
-                        const f2 DUDS = mul2(pk(0.5f, 0.5f), fma2(DS, RS, mul2(DR, RR)));
-                        float a0, b0, a1, b1;
-                        Lds<FMT>::pair(rowS + q0 * (unsigned)sizeof(T), a0, b0);
-                        Lds<FMT>::pair(rowS + q1 * (unsigned)sizeof(T), a1, b1);
-                        const f2 A = pk(a0, a1);
-                        const f2 DV = sub2(pk(b0, b1), A);
-                        f2 TERM;
-                        if (PRE == kWtPrefold) {
-                            TERM = DV;
-                        } else {
-                            const float2 w0 = lds_f2(wS + q0 * 8u), w1 = lds_f2(wS + q1 * 8u);
-                            const f2 DW = pk(w0.y, w1.y);
-                            const f2 W = fma2(F, DW, pk(w0.x, w1.x));
-                            const f2 V = fma2(F, DV, A);
-                            TERM = fma2(DW, V, mul2(W, DV));
-                        }
-                        acc[h] = fma2(mul2(SC, TERM), DUDS, acc[h]);
-                        continue;
-                    }
-                    const PairKin kk = pair_kin(DS, DR, S2[h], T2[h], umax, M2);
-                    const f2 F = kk.F;
-                    const float u0 = kk.u0, u1 = kk.u1;
-                    const unsigned q0 = kk.q0, q1 = kk.q1;
-                    const unsigned ad0 = rowS + q0 * (unsigned)sizeof(T);
-                    const unsigned ad1 = rowS + q1 * (unsigned)sizeof(T);
-                    f2 V;
-                    if (PICK == KTM_PICK_LINEAR) {
-                        float a0, b0, a1, b1;
-                        Lds<FMT>::pair(ad0, a0, b0);
-                        Lds<FMT>::pair(ad1, a1, b1);
-                        const f2 A = pk(a0, a1);
-                        V = fma2(F, sub2(pk(b0, b1), A), A);
-                    } else {
-                        V = pk(Lds<FMT>::one(ad0), Lds<FMT>::one(ad1));
-                    }
+                for (int d = H > 4 ? 4 : 2; kStepwise && d > 0; d >>= 1)
+                    if (hmax - 1 + d < H && reaches(hmax - 1 + d)) hmax += d;
+            }
+        }
+        const unsigned kept = __ballot_sync(0xffffffffu, hmax > 0);
+        const int cnt = __popc(kept);
+        // bits(fl) = kMagicBits + i0: fold the magic offset into the bases (mod 2^32)
+        const unsigned magicT = (unsigned)kMagicBits * (unsigned)sizeof(T);
+        const unsigned wS = smem_u32(smem_raw + L.wtabOff) - (unsigned)kMagicBits * 8u;
+        if (hmax > 0) {
+            // rows are 16-byte aligned: the steps go into the address's low bits
+            const unsigned row = smem_u32(smem_raw) + (unsigned)(b * L.rawBytes) +
+                                 (unsigned)(lane * a.pitch) * (unsigned)sizeof(T) - magicT;
+            tab[__popc(kept & ((1u << lane) - 1u))] = make_float4(ds, dr, sc, __uint_as_float(row + (unsigned)hmax));
+        }
+        __syncwarp();
+        keptTraces += (unsigned)cnt;
+        // the ch/stages-th use of buffer b completes that phase of its barrier
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&cs.bar[b], (unsigned)parity, kBulkWaitNs))) {
+            if (lane == 0) {
+                cs.stalled = 1;
+                atomicAdd(&g_waitStalls, 1u);
+            }
+            break;
+        }
+        for (int e = 0; e < cnt; e++) {
+            const float4 t = tab[e];
+            const unsigned rowBits = __float_as_uint(t.w);
+            const int hm = (int)(rowBits & 15u);
+            const unsigned rowS = rowBits & ~15u;
+            const f2 DS = pk(t.x, t.x), DR = pk(t.y, t.y), SC = pk(t.z, t.z);
+            // step h: two tau samples of each lane
+            auto pairs = [&](int h) __attribute__((always_inline)) {
+                if (GRAD) {
+                    // d/dS' of |tau| s_k W(u) V(u), u = sqrt(a_s) + sqrt(a_r):
+                    // (dW/du V + W dV/du) du/dS', du/dS' = Ds/(2 sqrt a_s) + Dr/(2 sqrt a_r)
+                    float as0, as1, ar0, ar1;
+                    upk(fma2(DS, S2[h], T2[h]), as0, as1);
+                    upk(fma2(DR, S2[h], T2[h]), ar0, ar1);
+                    const f2 RS = pk(fminf(rsqrt_approx(as0), 3.0e38f), fminf(rsqrt_approx(as1), 3.0e38f));
+                    const f2 RR = pk(fminf(rsqrt_approx(ar0), 3.0e38f), fminf(rsqrt_approx(ar1), 3.0e38f));
+                    f2 U = fma2(pk(ar0, ar1), RR, mul2(pk(as0, as1), RS));
+                    float u0, u1;
+                    upk(U, u0, u1);
+                    u0 = fminf(u0, umax);
+                    u1 = fminf(u1, umax);
+                    U = pk(u0, u1);
+                    const f2 FL = add2_rm(U, M2);
+                    float fl0, fl1;
+                    upk(FL, fl0, fl1);
+                    const unsigned q0 = __float_as_uint(fl0), q1 = __float_as_uint(fl1);
+                    const f2 F = sub2(U, sub2(FL, M2));
+                    const f2 DUDS = mul2(pk(0.5f, 0.5f), fma2(DS, RS, mul2(DR, RR)));
+                    float a0, b0, a1, b1;
+                    Lds<FMT>::pair(rowS + q0 * (unsigned)sizeof(T), a0, b0);
+                    Lds<FMT>::pair(rowS + q1 * (unsigned)sizeof(T), a1, b1);
+                    const f2 A = pk(a0, a1);
+                    const f2 DV = sub2(pk(b0, b1), A);
+                    f2 TERM;
                     if (PRE == kWtPrefold) {
-                        acc[h] = fma2(SC, V, acc[h]);
-                    } else if (PRE == kWtTable) {
-                        const float2 w0 = lds_f2(wS + q0 * 8u), w1 = lds_f2(wS + q1 * 8u);
-                        const f2 W = fma2(F, pk(w0.y, w1.y), pk(w0.x, w1.x));
-                        acc[h] = fma2(mul2(SC, W), V, acc[h]);
+                        TERM = DV;
                     } else {
-                        // u is in samples: sqrt(t) = sqrt(u) sqrt(dt), sqrt(dt) applied at the end
-                        const f2 W = pk(sqrt_approx(u0), sqrt_approx(u1));
-                        acc[h] = fma2(mul2(SC, W), V, acc[h]);
+                        const float2 w0 = lds_f2(wS + q0 * 8u), w1 = lds_f2(wS + q1 * 8u);
+                        const f2 DW = pk(w0.y, w1.y);
+                        const f2 W = fma2(F, DW, pk(w0.x, w1.x));
+                        const f2 V = fma2(F, DV, A);
+                        TERM = fma2(DW, V, mul2(W, DV));
                     }
+                    acc[h] = fma2(mul2(SC, TERM), DUDS, acc[h]);
+                    return;
+                }
+                const PairKin kk = pair_kin(DS, DR, S2[h], T2[h], umax, M2);
+                const f2 F = kk.F;
+                const float u0 = kk.u0, u1 = kk.u1;
+                const unsigned q0 = kk.q0, q1 = kk.q1;
+                const unsigned ad0 = rowS + q0 * (unsigned)sizeof(T);
+                const unsigned ad1 = rowS + q1 * (unsigned)sizeof(T);
+                f2 V;
+                if (PICK == KTM_PICK_LINEAR) {
+                    float a0, b0, a1, b1;
+                    Lds<FMT>::pair(ad0, a0, b0);
+                    Lds<FMT>::pair(ad1, a1, b1);
+                    const f2 A = pk(a0, a1);
+                    V = fma2(F, sub2(pk(b0, b1), A), A);
+                } else {
+                    V = pk(Lds<FMT>::one(ad0), Lds<FMT>::one(ad1));
+                }
+                if (PRE == kWtPrefold) {
+                    acc[h] = fma2(SC, V, acc[h]);
+                } else if (PRE == kWtTable) {
+                    const float2 w0 = lds_f2(wS + q0 * 8u), w1 = lds_f2(wS + q1 * 8u);
+                    const f2 W = fma2(F, pk(w0.y, w1.y), pk(w0.x, w1.x));
+                    acc[h] = fma2(mul2(SC, W), V, acc[h]);
+                } else {
+                    // u is in samples: sqrt(t) = sqrt(u) sqrt(dt), sqrt(dt) applied at the end
+                    const f2 W = pk(sqrt_approx(u0), sqrt_approx(u1));
+                    acc[h] = fma2(mul2(SC, W), V, acc[h]);
+                }
+            };
+            // all steps in one block the compiler interleaves, or step by step up to the last
+            // one that reaches the trace end
+            if (!kStepwise || hm == H) {
+#pragma unroll
+                for (int h = 0; h < H; h++) pairs(h);
+            } else {
+#pragma unroll
+                for (int h = 0; h < H; h++) {
+                    if (h > 0 && h >= hm) break;
+                    pairs(h);
                 }
             }
+        }
+        // the last warp through with the chunk starts the copy of the one that follows in
+        // this buffer
+        __syncwarp();
+        if (lane == 0) {
+            __threadfence_block();
+            if (atomicAdd(&cs.done[b], 1) == active - 1) {
+                cs.done[b] = 0;
+                __threadfence_block();
+                if (ch + st.stages < nchunks) issue(ch + st.stages, b);
+            }
+        }
+        if (++b == st.stages) {
+            b = 0;
+            parity ^= 1;
         }
     }
 
+    __syncthreads();
     if (threadIdx.x == 0) {
-        mbar_inval(&cs.bar[0]);
-        mbar_inval(&cs.bar[1]);
+        for (int b = 0; b < st.stages; b++) {
+            // a tile that gave up waits (bounded) for its copies in flight
+            if (cs.stalled && cs.issued[b]) mbar_wait_bounded(&cs.bar[b], (unsigned)(cs.issued[b] - 1) & 1u, kBulkWaitNs);
+            mbar_inval(&cs.bar[b]);
+        }
     }
+    if (cs.stalled) return false;              // CTA-uniform: no output from this tile
     if (colValid) {
         float* out = (outMode == kOutPartial ? partial : a.image) + (size_t)col * g.nz;
 #pragma unroll
@@ -389,7 +454,7 @@ struct BatchTile {
 
 template <class SH, int R, int PICK, int FMT, int PRE>
 __global__ void __launch_bounds__(SH::kThreads, SH::kMinBlocks)
-batch_kernel(const FastArgs* __restrict__ jobs, const int* __restrict__ chunks,
+batch_kernel(const FastArgs* __restrict__ jobs, const Stages* __restrict__ chunks,
              const BatchTile* __restrict__ tiles, int ntiles, unsigned* __restrict__ counter)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -416,14 +481,14 @@ batch_kernel(const FastArgs* __restrict__ jobs, const int* __restrict__ chunks,
 
 template <class SH, int R, int PICK, int FMT, int PRE, int GRAD>
 __global__ void __launch_bounds__(SH::kThreads, SH::kMinBlocks)
-fast_kernel(FastArgs a, int chunk, int perSlice, float* __restrict__ partial)
+fast_kernel(FastArgs a, Stages st, int perSlice, float* __restrict__ partial)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ ChunkSync cs;
     const int kb = blockIdx.z * perSlice;
     const int ke = min(a.g.ntr, kb + perSlice);
     const size_t nimg = (size_t)a.g.nx * a.g.ny * a.g.nz;
-    fast_tile<SH, R, PICK, FMT, PRE, GRAD>(a, chunk, blockIdx.x, blockIdx.y, kb, ke,
+    fast_tile<SH, R, PICK, FMT, PRE, GRAD>(a, st, blockIdx.x, blockIdx.y, kb, ke,
                                        partial ? partial + blockIdx.z * nimg : nullptr,
                                        partial ? kOutPartial : kOutImage, smem_raw, cs);
 }
@@ -440,19 +505,52 @@ __global__ void reduce_slices(float* __restrict__ out, const float* __restrict__
     }
 }
 
-// Traces per chunk: as many as the shape's shared-memory budget holds (at most
-// kMaxChunk), or fewer when the caller caps them (chunkCap > 0).  0 when even one
-// trace exceeds the largest allocation a CTA can have.
+// Traces per row buffer and buffers: as many traces as the shape's shared-memory budget
+// holds (at most kMaxChunk per buffer, or fewer when the caller caps them: chunkCap > 0),
+// in three buffers where each still gets 16 traces, else in two: the third lets the warps
+// drift further apart, fewer traces per buffer cost more of the per-chunk geometry.  chunk 0
+// for traces beyond the limit: two of them, with the weight table, exceed the largest
+// allocation a CTA can have.
 template <class SH>
-int fast_chunk(const FastArgs& a, int esize, bool table)
+Stages fast_stages(const FastArgs& a, int esize, bool table)
 {
-    int chunk = kMaxChunk;
-    if (a.chunkCap > 0) chunk = std::min(chunk, a.chunkCap);
-    while (chunk > 1 && chunk_layout(chunk, a.pitch, esize, a.g.nt, table).total > SH::kBudget)
-        chunk--;
-    if (chunk_layout(chunk, a.pitch, esize, a.g.nt, table).total > (size_t)kMaxSmemBytes)
-        return 0;
-    return chunk;
+    const int cap = a.chunkCap > 0 ? std::min(kMaxChunk, a.chunkCap) : kMaxChunk;
+    auto fit = [&](int stages) {
+        Stages s = {cap, stages};
+        while (s.chunk > 1 && chunk_layout(s, SH::kWarps, a.pitch, esize, a.g.nt, table).total > SH::kBudget)
+            s.chunk--;
+        return s;
+    };
+    // two buffers of one trace and its 48 bytes of coordinates beside the table
+    if (2 * (size_t)a.pitch * esize + 48 + (table ? (a.g.nt + 1) * sizeof(float2) : 0) > (size_t)kMaxSmemBytes)
+        return Stages{0, 0};
+    Stages s = fit(3);
+    if (s.chunk < std::min(cap, 16)) s = fit(2);
+    // the longest traces: two buffers leave no room for the warps' tables
+    if (chunk_layout(s, SH::kWarps, a.pitch, esize, a.g.nt, table).total > (size_t)kMaxSmemBytes) s.stages = 1;
+    return s;
+}
+
+// Trace slices of a launch of `base` CTAs per slice on `slots` resident CTAs: the number
+// with the least estimated time, in traces of a CTA: a CTA takes its traces + 8 for its
+// prologue; up to `slots` of them run at once, more end unevenly (aperture, trace end), half a
+// CTA past the mean; plus the partial images (a trace takes about 1 us at R = 16, 6.5 MB of
+// partial images the same).
+int choose_slices(long long base, int slots, int ntr, int R, size_t nimg, int most)
+{
+    int best = 1;
+    float least = 3.0e38f;
+    for (int s = 1; s <= most; s++) {
+        const float per = (float)((ntr + s - 1) / s) + 8.0f;
+        const float rounds = base * s <= slots ? 1.0f : (float)(base * s) / (float)slots + 0.5f;
+        const float copies = s > 1 ? (float)s * (float)nimg * (8.0f / 6.5e6f) * 16.0f / (float)R : 0.0f;
+        const float cost = rounds * per + copies;
+        if (cost < least) {
+            least = cost;
+            best = s;
+        }
+    }
+    return best;
 }
 
 // One grid launch over all of a's traces.
@@ -462,11 +560,12 @@ int launch_block(const FastArgs& a, cudaStream_t stream, int smCount)
     const Geometry& g = a.g;
     const int esize = FMT == KTM_FMT_F32 ? 4 : 2;
     constexpr bool kTable = PRE == kWtTable;
-    const int chunk = fast_chunk<SH>(a, esize, kTable);
+    const Stages st = fast_stages<SH>(a, esize, kTable);
+    const int chunk = st.chunk;
     if (chunk == 0)
         return set_error(KTM_ERR_LIMIT, "fast kernel: packed pitch %d exceeds the shared-memory "
                                         "stage limit", a.pitch);
-    const size_t smem = chunk_layout(chunk, a.pitch, esize, g.nt, kTable).total;
+    const size_t smem = chunk_layout(st, SH::kWarps, a.pitch, esize, g.nt, kTable).total;
     auto kern = fast_kernel<SH, R, PICK, FMT, PRE, GRAD>;
     KTM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 
@@ -474,19 +573,15 @@ int launch_block(const FastArgs& a, cudaStream_t stream, int smCount)
     const unsigned gx = (unsigned)((cols + SH::kWarps - 1) / SH::kWarps);
     const unsigned gy = (unsigned)((g.nz + 32 * R - 1) / (32 * R));
     if (gy > 65535) return set_error(KTM_ERR_LIMIT, "fast kernel: Nz too large");
-    // trace slices: about eight CTAs per SM over the launch, each slice keeping at
-    // least four chunks of traces
-    const long long base = (long long)gx * gy;
-    const long long want = 8LL * smCount;
-    int slices = (int)((want + base - 1) / base);
-    const int maxSlices = max(1, g.ntr / (4 * chunk));
-    slices = max(1, min(slices, min(maxSlices, 64)));
-    if (a.slices > 0) slices = min(a.slices, max(1, g.ntr));
+    const size_t nimg = (size_t)cols * g.nz;
+    // at least eight traces to a slice, at most 64 slices
+    int slices = a.slices > 0 ? min(a.slices, max(1, g.ntr))
+                              : choose_slices((long long)gx * gy, SH::kMinBlocks * smCount, g.ntr, R, nimg,
+                                              max(1, min(64, g.ntr / 8)));
     const int perSlice = (g.ntr + slices - 1) / slices;
     slices = (g.ntr + perSlice - 1) / perSlice;
 
     float* partial = nullptr;
-    const size_t nimg = (size_t)cols * g.nz;
     if (slices > 1) {
         if (a.scratch && a.scratchBytes >= (size_t)slices * nimg * sizeof(float)) {
             partial = static_cast<float*>(a.scratch);
@@ -496,7 +591,7 @@ int launch_block(const FastArgs& a, cudaStream_t stream, int smCount)
         }
     }
     dim3 grid(gx, gy, (unsigned)slices);
-    kern<<<grid, SH::kThreads, smem, stream>>>(a, chunk, perSlice, partial);
+    kern<<<grid, SH::kThreads, smem, stream>>>(a, st, perSlice, partial);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && partial) {
         const int th = 256;
@@ -735,16 +830,16 @@ int launch_batch_t(const FastArgs* jobs, int njobs, cudaStream_t s)
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
     const int ctas = SH::kMinBlocks * sm;
-    std::vector<int> chunks(njobs);
+    std::vector<Stages> chunks(njobs);
     size_t smem = 0;
     double totalPairs = 0.0;
     for (int j = 0; j < njobs; j++) {
         const Geometry& g = jobs[j].g;
-        const int c = fast_chunk<SH>(jobs[j], esize, PRE == kWtTable);
-        if (c == 0)
+        const Stages c = fast_stages<SH>(jobs[j], esize, PRE == kWtTable);
+        if (c.chunk == 0)
             return set_error(KTM_ERR_LIMIT, "batch: job %d packed pitch %d exceeds shared memory", j,
                              jobs[j].pitch);
-        const size_t need = chunk_layout(c, jobs[j].pitch, esize, g.nt, PRE == kWtTable).total;
+        const size_t need = chunk_layout(c, SH::kWarps, jobs[j].pitch, esize, g.nt, PRE == kWtTable).total;
         chunks[j] = c;
         smem = std::max(smem, need);
         totalPairs += (double)g.nx * g.ny * g.nz * g.ntr;
@@ -761,7 +856,7 @@ int launch_batch_t(const FastArgs* jobs, int njobs, cudaStream_t s)
         const int cgs = (int)((cols + SH::kWarps - 1) / SH::kWarps);
         const int runs = (g.nz + 32 * R - 1) / (32 * R);
         const double tilePairsPerTrace = (double)SH::kWarps * 32 * R;
-        int per = (int)std::min<double>(g.ntr, std::max<double>(4.0 * chunks[j], perTile / tilePairsPerTrace));
+        int per = (int)std::min<double>(g.ntr, std::max<double>(4.0 * chunks[j].chunk, perTile / tilePairsPerTrace));
         per = std::max(per, 1);
         for (int cg = 0; cg < cgs; cg++)
             for (int r = 0; r < runs; r++)
@@ -784,13 +879,13 @@ int launch_batch_t(const FastArgs* jobs, int njobs, cudaStream_t s)
     std::vector<BatchTile> sorted(tiles.size());
     for (size_t i = 0; i < order.size(); i++) sorted[i] = tiles[order[i]];
 
-    const size_t bJobs = sizeof(FastArgs) * njobs, bChunks = sizeof(int) * njobs;
+    const size_t bJobs = sizeof(FastArgs) * njobs, bChunks = sizeof(Stages) * njobs;
     const size_t bTiles = sizeof(BatchTile) * sorted.size();
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
     unsigned char* buf = nullptr;
     KTM_CUDA_TRY(pool_malloc(reinterpret_cast<void**>(&buf), up(bJobs) + up(bChunks) + up(bTiles) + 256, s));
     FastArgs* dJobs = reinterpret_cast<FastArgs*>(buf);
-    int* dChunks = reinterpret_cast<int*>(buf + up(bJobs));
+    Stages* dChunks = reinterpret_cast<Stages*>(buf + up(bJobs));
     BatchTile* dTiles = reinterpret_cast<BatchTile*>(buf + up(bJobs) + up(bChunks));
     unsigned* dCounter = reinterpret_cast<unsigned*>(buf + up(bJobs) + up(bChunks) + up(bTiles));
     cudaError_t e = cudaMemcpyAsync(dJobs, jobs, bJobs, cudaMemcpyHostToDevice, s);
