@@ -24,6 +24,7 @@
 #include "ktm_pair.cuh"
 
 #include <algorithm>
+#include <cstring>
 
 namespace ktm {
 namespace {
@@ -273,19 +274,381 @@ demigrate_merge_kernel(AdjArgs a)
     }
 }
 
+// ---------------------------------------------------------------------------
+// Demigration with a row per warp: linear pick, 1-D velocity, traces short enough that
+// sixteen rows fit an SM.
+//
+// A warp owns one trace (of the column block blockIdx.y): it accumulates the trace into a
+// row of its own in shared memory while it sweeps runs of 256 tau samples and, for each run,
+// the columns, lane c evaluating 32 columns' geometry at a time.  T2', S' of the run stay in
+// registers over all columns (1-D velocity); |tau| m comes from a copy that a first kernel
+// laid out so that a lane's 8 samples are two 16-byte loads (zero runs are flagged there).
+//
+// No other warp writes the row, so where two lanes cannot meet either, a flush is a plain
+// load, add and store instead of a compare-and-swap loop.  Lane L owns samples 8 L .. 8 L + 7
+// of the run and flushes sample floor(u) when u leaves it.  With all 8 indices at hand the
+// warp looks whether in every lane floor(u) stays or goes on by one from each sample to the
+// next, and whether the next lane is ahead at every step (past the trace end they may meet:
+// those words are dropped).  If so each step's flushes hit different words, and one
+// comparison a sample does the merge.  Elsewhere (shallow runs, where 8 samples may share a
+// trace sample; steep steps) it takes the merge of demigrate_merge_kernel with shared
+// reductions.
+// 512 x 1001 image, 32,768 traces of 1001 samples, prefolded / table / sqrt weight:
+// 11.4 / 18.0 / 12.5 ms, against 14.7 / 18.5 / 15.4 with rows shared by the CTA; 100 columns,
+// 2000 traces 0.33 / 0.47 against 0.54 / 0.59.  Bound by issue (35 instructions a pair, three
+// quarters of the slots) and by the shared-memory pipe.
+constexpr int kRowR = 8;
+constexpr int kRowRun = 32 * kRowR;
+// Warps per CTA, up to 32 warps per SM: small CTAs end at their own pace (512 x 1001 image,
+// 32,768 traces, prefolded: 11.3 ms in CTAs of 8 warps, 12.2 in CTAs of 32); with the weight
+// table, of which every CTA holds a copy, 16 (18.7 ms in CTAs of 8, 18.0 in CTAs of 16).
+template <int WT>
+constexpr int kRowWarps = WT == 0 ? 16 : 8;
+
+struct RowArgs {
+    AdjArgs a;
+    const float* mt;              // |tau| m, [ncols][nruns][2][32][4]
+    const unsigned char* live;    // [ncols][nruns]: a sample of the run is not zero
+    int nruns, accumulate;
+};
+
+__host__ __device__ __forceinline__ int row_words(int nt) { return padded_pitch(nt + 2); }
+
+// |tau| m and the non-zero flags, one warp per (column, run)
+__global__ void __launch_bounds__(256) row_model_kernel(AdjArgs a, int nruns, float* __restrict__ mt,
+                                                        unsigned char* __restrict__ live)
+{
+    const Geometry& g = a.g;
+    const int lane = threadIdx.x & 31;
+    const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (w >= (long long)g.nx * g.ny * nruns) return;
+    const long long col = w / nruns;
+    const int run = (int)(w - col * nruns);
+    bool any = false;
+#pragma unroll
+    for (int i = 0; i < kRowR; i++) {
+        const int x = 32 * i + lane;                       // sample of the run
+        const int l = run * kRowRun + x;
+        const float tau = g.z0 + (float)l * g.dz;
+        const float v = l < g.nz ? fabsf(tau) * a.image[col * g.nz + l] : 0.0f;
+        any |= v != 0.0f;
+        // lane x / 8, half (x / 4) % 2, word x % 4
+        mt[w * kRowRun + ((x >> 2) & 1) * 128 + (x >> 3) * 4 + (x & 3)] = v;
+    }
+    any = __any_sync(0xffffffffu, any);
+    if (lane == 0) live[w] = any;
+}
+
+// T2' and S' of tau sample l: past the image T2' goes on and S' stays
+__device__ __forceinline__ void row_tables(const AdjArgs& a, int l, float invdt, float& t2, float& s)
+{
+    const Geometry& g = a.g;
+    const float tq = (g.z0 + (float)l * g.dz) * invdt;
+    const float vd = a.vel[l < g.nz ? l : g.nz - 1] * g.dt;
+    t2 = tq * tq;
+    s = 1.0f / (vd * vd);
+}
+
+// row[addr] += v where `on` holds: predicated, so the warp stays converged
+__device__ __forceinline__ void add_shared_if(bool on, unsigned addr, float v)
+{
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .f32 t;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.shared.f32 t, [%0];\n\t"
+                 "@p add.f32 t, t, %1;\n\t@p st.shared.f32 [%0], t;\n\t}"
+                 ::"r"(addr), "f"(v), "r"((unsigned)on));
+}
+__device__ __forceinline__ void add_shared(unsigned addr, float v)
+{
+    asm volatile("{\n\t.reg .f32 t;\n\tld.shared.f32 t, [%0];\n\tadd.f32 t, t, %1;\n\tst.shared.f32 [%0], t;\n\t}"
+                 ::"r"(addr), "f"(v));
+}
+
+// word (in bytes) of the sample whose bits(fl) = q, relative to the row's shifted base
+__device__ __forceinline__ unsigned padded_bytes(unsigned q) { return (q + (q >> kPadShift)) * 4u; }
+
+template <int WT>
+__global__ void __launch_bounds__(kRowWarps<WT> * 32, 32 / kRowWarps<WT>) demigrate_row_kernel(RowArgs ra)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const AdjArgs& a = ra.a;
+    const Geometry& g = a.g;
+    constexpr int warps = kRowWarps<WT>;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int words = row_words(g.nt);
+    // [warps] rows, [warps][32] entries, [nruns] least T2' and S', the padded weight table
+    float* row = reinterpret_cast<float*>(smem_raw) + (size_t)warp * words;
+    float4* tab = reinterpret_cast<float4*>(smem_raw + (size_t)warps * words * 4) + warp * 32;
+    float2* least = reinterpret_cast<float2*>(smem_raw + (size_t)warps * (words * 4 + 512));
+    float2* wtab = least + (ra.nruns + 1) / 2 * 2;
+    const float invdt = 1.0f / g.dt;
+
+    for (int i = lane; i < words; i += 32) row[i] = 0.0f;
+    for (int run = warp; run < ra.nruns; run += warps) {
+        float t2 = 3.0e38f, sl = 3.0e38f;
+        for (int i = 0; i < kRowR; i++) {
+            const int l = run * kRowRun + 32 * i + lane;
+            float t0, s0;
+            row_tables(a, l, invdt, t0, s0);
+            if (l < g.nz) {
+                t2 = fminf(t2, t0);
+                sl = fminf(sl, s0);
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            t2 = fminf(t2, __shfl_xor_sync(0xffffffffu, t2, o));
+            sl = fminf(sl, __shfl_xor_sync(0xffffffffu, sl, o));
+        }
+        if (lane == 0) least[run] = make_float2(t2, sl);
+    }
+    if (WT == 0) {
+        for (int j = threadIdx.x; j <= g.nt; j += blockDim.x) {
+            const float w0 = sqrtf((float)j * g.dt), w1 = sqrtf((float)(j + 1) * g.dt);
+            wtab[j + (j >> kPadShift)] = make_float2(w0, w1 - w0);
+        }
+    }
+    __syncthreads();
+
+    const int k = blockIdx.x * warps + warp;
+    if (k >= g.ntr) return;
+    const float mx = a.midX[k], my = a.midY[k], ox = a.offX[k], oy = a.offY[k];
+    const int cb0 = blockIdx.y * a.colsPerBlock, cb1 = min(g.nx * g.ny, cb0 + a.colsPerBlock);
+    const float umax = (float)g.nt, upast = umax * 1.0001f + 1.0f;
+    const float ap2 = a.aperture > 0.0f ? a.aperture * a.aperture : -1.0f;
+    const f2 M2 = pk(kMagic, kMagic);
+    // bits(fl) = K + i0, K a multiple of 4: the bases carry -padded(K)
+    const unsigned kPad = (unsigned)kMagicBits + ((unsigned)kMagicBits >> kPadShift);
+    const unsigned rowS = smem_u32(row) - kPad * 4u;
+    const unsigned wS = smem_u32(wtab) - kPad * 8u;
+    const unsigned qEnd = (unsigned)kMagicBits + (unsigned)g.nt;
+    const float rootDt = sqrtf(g.dt);
+
+    for (int run = 0; run < ra.nruns; run++) {
+        f2 T2[kRowR / 2], S2[kRowR / 2];
+#pragma unroll
+        for (int h = 0; h < kRowR / 2; h++) {
+            float t[2], s[2];
+#pragma unroll
+            for (int e = 0; e < 2; e++) row_tables(a, run * kRowRun + kRowR * lane + 2 * h + e, invdt, t[e], s[e]);
+            T2[h] = pk(t[0], t[1]);
+            S2[h] = pk(s[0], s[1]);
+        }
+        for (int cb = cb0; cb < cb1; cb += 32) {
+            // lane c: column cb + c
+            float ds = 0.0f, dr = 0.0f;
+            bool keep = false;
+            const int col = cb + lane;
+            if (col < cb1) {
+                const int ci = col / g.ny, cj = col - ci * g.ny;
+                const float dmx = mx - (g.x0 + (float)ci * g.dx), dmy = my - (g.y0 + (float)cj * g.dy);
+                const float sx = dmx - ox, sy = dmy - oy, rx = dmx + ox, ry = dmy + oy;
+                ds = sx * sx + sy * sy;
+                dr = rx * rx + ry * ry;
+                // aperture, a zero model, a first sample past the trace end
+                const float2 m = least[run];
+                keep = !(ap2 >= 0.0f && dmx * dmx + dmy * dmy > ap2) && ra.live[(size_t)col * ra.nruns + run] &&
+                       sqrt_approx(fmaf(ds, m.y, m.x)) + sqrt_approx(fmaf(dr, m.y, m.x)) < upast;
+            }
+            const unsigned kept = __ballot_sync(0xffffffffu, keep);
+            if (keep) tab[__popc(kept & ((1u << lane) - 1u))] = make_float4(ds, dr, __int_as_float(col), 0.0f);
+            __syncwarp();
+            const int cnt = __popc(kept);
+            for (int e = 0; e < cnt; e++) {
+                const float4 t = tab[e];
+                const float4* m4 = reinterpret_cast<const float4*>(
+                    ra.mt + ((size_t)__float_as_int(t.z) * ra.nruns + run) * kRowRun) + lane;
+                const float4 ma = __ldg(m4), mb = __ldg(m4 + 32);
+                const f2 DS = pk(t.x, t.x), DR = pk(t.y, t.y);
+                const f2 MT[4] = {pk(ma.x, ma.y), pk(ma.z, ma.w), pk(mb.x, mb.y), pk(mb.z, mb.w)};
+                unsigned q[kRowR];
+                float ca[kRowR], cb_[kRowR];       // to samples floor(u) and floor(u) + 1
+#pragma unroll
+                for (int h = 0; h < kRowR / 2; h++) {
+                    const PairKin kk = pair_kin(DS, DR, S2[h], T2[h], umax, M2);
+                    q[2 * h] = kk.q0;
+                    q[2 * h + 1] = kk.q1;
+                    f2 VAL = MT[h];
+                    if (WT == 0) {
+                        const float2 w0 = lds_f2(wS + 2u * padded_bytes(kk.q0)), w1 = lds_f2(wS + 2u * padded_bytes(kk.q1));
+                        VAL = mul2(fma2(kk.F, pk(w0.y, w1.y), pk(w0.x, w1.x)), MT[h]);
+                    } else if (WT == 1) {
+                        VAL = mul2(mul2(pk(sqrt_approx(kk.u0), sqrt_approx(kk.u1)), pk(rootDt, rootDt)), MT[h]);
+                    }
+                    const f2 B = mul2(VAL, kk.F);          // f * val       -> sample i0 + 1
+                    const f2 A = sub2(VAL, B);             // (1 - f) * val -> sample i0
+                    upk(A, ca[2 * h], ca[2 * h + 1]);
+                    upk(B, cb_[2 * h], cb_[2 * h + 1]);
+                }
+                // steps of at most one sample; the next lane ahead (the last lane has none)
+                bool small = true, apart = true;
+#pragma unroll
+                for (int i = 0; i < kRowR; i++) {
+                    const unsigned n = __shfl_down_sync(0xffffffffu, q[i], 1);
+                    apart = apart && (n > q[i] || n == qEnd || lane == 31);
+                    if (i > 0) small = small && q[i] - q[i - 1] <= 1u;
+                }
+                small = __all_sync(0xffffffffu, small);
+                float va = ca[0], vb = cb_[0];
+                if (__all_sync(0xffffffffu, apart) && small) {
+#pragma unroll
+                    for (int i = 1; i < kRowR; i++) {
+                        const bool on = q[i] != q[i - 1];
+                        add_shared_if(on, rowS + padded_bytes(q[i - 1]), va);
+                        va = (on ? vb : va) + ca[i];
+                        vb = (on ? 0.0f : vb) + cb_[i];
+                        __syncwarp();
+                    }
+                    add_shared(rowS + padded_bytes(q[kRowR - 1]), va);
+                    __syncwarp();
+                    add_shared(rowS + padded_bytes(q[kRowR - 1] + 1u), vb);
+                    __syncwarp();
+                } else if (small) {
+#pragma unroll
+                    for (int i = 1; i < kRowR; i++) {
+                        const bool on = q[i] != q[i - 1];
+                        red_shared_if(on, rowS + padded_bytes(q[i - 1]), va);
+                        va = (on ? vb : va) + ca[i];
+                        vb = (on ? 0.0f : vb) + cb_[i];
+                    }
+                    red_shared(rowS + padded_bytes(q[kRowR - 1]), va);
+                    red_shared(rowS + padded_bytes(q[kRowR - 1] + 1u), vb);
+                    __syncwarp();
+                } else {
+#pragma unroll
+                    for (int i = 1; i < kRowR; i++) {
+                        const unsigned qc = q[i - 1];
+                        const bool same = q[i] == qc, next = q[i] == qc + 1u;
+                        red_shared_if(!same, rowS + padded_bytes(qc), va);
+                        red_shared_if(!same && !next, rowS + padded_bytes(qc + 1u), vb);
+                        va = same ? va + ca[i] : (next ? vb + ca[i] : ca[i]);
+                        vb = same ? vb + cb_[i] : cb_[i];
+                    }
+                    red_shared(rowS + padded_bytes(q[kRowR - 1]), va);
+                    red_shared(rowS + padded_bytes(q[kRowR - 1] + 1u), vb);
+                    __syncwarp();
+                }
+            }
+        }
+    }
+    asm volatile("" ::: "memory");     // the scatter wrote the row: no load below reuses older values
+    __syncwarp();
+    float* dst = a.data + (size_t)k * a.pitch;
+    for (int j = lane; j < a.pitch; j += 32) {
+        float v = (j > 0 && j < g.nt) ? row[j + (j >> kPadShift)] : 0.0f;
+        if (WT == 2) v *= sqrtf((float)j * g.dt);        // the fold's factor (ktm_prep.cu, ktm_lsm.cu)
+        if (a.atomicOut) {
+            if (v != 0.0f) atomicAdd(dst + j, v);
+        } else {
+            dst[j] = ra.accumulate ? dst[j] + v : v;
+        }
+    }
+}
+
+// Shared memory of a CTA of the row kernel, and how many fit an SM; 0: the job takes the
+// shared rows.  Sixteen warps an SM are enough for it (2201 samples: 11.8 ms against 13.4)
+// except with the weight table (1501 samples, 16 warps: 29.2 ms against 28.4) and with tau
+// steps of more than half a sample, which make most flushes general ones (2201 samples, 16
+// warps, 41.0 ms against 28.6; 1001 samples, 32 warps, 10.8 against 10.8; 500 samples 5.3
+// against 7.0): those need 32, and never take it both with the table and coarse steps (16.6
+// ms against 15.4).
+int row_ctas(const Geometry& g, int wt, size_t* smem)
+{
+    const int nruns = (g.nz + kRowRun - 1) / kRowRun, warps = wt == 0 ? kRowWarps<0> : kRowWarps<1>;
+    *smem = warps * ((size_t)row_words(g.nt) * 4 + 512) + (nruns + 1) / 2 * 16 +
+            (wt == 0 ? (size_t)padded_pitch(g.nt + 1) * sizeof(float2) : 0);
+    const int ctas = (int)std::min<size_t>(32 / warps, (size_t)(227 * 1024) / (*smem + 1024));
+    const bool coarse = !(2.0f * fabsf(g.dz) <= 1.05f * g.dt);
+    if (g.nt > 8192 || (wt == 0 && coarse)) return 0;
+    return ctas * warps >= (wt == 0 || coarse ? 32 : 16) ? ctas : 0;
+}
+
+template <int WT>
+int launch_rows(const RowArgs& ra, dim3 grid, size_t smem, cudaStream_t s)
+{
+    KTM_CUDA_TRY(cudaFuncSetAttribute(demigrate_row_kernel<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    demigrate_row_kernel<WT><<<grid, kRowWarps<WT> * 32, smem, s>>>(ra);
+    KTM_CUDA_TRY(cudaGetLastError());
+    return KTM_OK;
+}
+
+}  // namespace
+
+size_t demigrate_scratch(const Geometry& g, int velCube, int pick, int weightMethod)
+{
+    const int wt = weightMethod == KTM_WEIGHT_SQRT ? 1 : weightMethod == KTM_WEIGHT_PREFOLD ? 2 : 0;
+    size_t smem;
+    if (velCube || pick != KTM_PICK_LINEAR || row_ctas(g, wt, &smem) == 0) return 0;
+    const size_t items = (size_t)g.nx * g.ny * ((g.nz + kRowRun - 1) / kRowRun);
+    return items * kRowRun * sizeof(float) + (items + 255) / 256 * 256;
+}
+
+namespace {
+
+// The row kernel over all traces: one CTA per kRowWarps traces and column block.
+int launch_row_demigrate(const Geometry& g, const float* midX, const float* midY, const float* offX,
+                         const float* offY, const float* vel, const float* image, float* data, int pitch,
+                         int weightMethod, float aperture, int accumulate, void* scratch, int sm, cudaStream_t s)
+{
+    const int wt = weightMethod == KTM_WEIGHT_SQRT ? 1 : weightMethod == KTM_WEIGHT_PREFOLD ? 2 : 0;
+    size_t smem = 0;
+    row_ctas(g, wt, &smem);
+    const int ncols = g.nx * g.ny, warps = wt == 0 ? kRowWarps<0> : kRowWarps<1>;
+    const int groups = (g.ntr + warps - 1) / warps;
+    // column blocks where the traces alone give too few CTAs, as many as the shared rows take
+    // (six groups of 32 traces per SM), so that both sum the same blocks of columns
+    const int chunks = (g.ntr + 31) / 32, want = 6 * sm;
+    int blocks = chunks < want ? std::min((want + chunks - 1) / chunks, std::max(1, ncols / 16)) : 1;
+    const int perBlock = (ncols + blocks - 1) / blocks;
+    blocks = (ncols + perBlock - 1) / perBlock;
+    RowArgs ra;
+    std::memset(&ra, 0, sizeof(ra));
+    AdjArgs& a = ra.a;
+    a.g = g; a.midX = midX; a.midY = midY; a.offX = offX; a.offY = offY;
+    a.vel = vel; a.image = image; a.data = data; a.pitch = pitch; a.aperture = aperture;
+    a.colsPerBlock = perBlock; a.atomicOut = blocks > 1;
+    ra.nruns = (g.nz + kRowRun - 1) / kRowRun;
+    ra.accumulate = accumulate;
+    const size_t items = (size_t)ncols * ra.nruns;
+    float* mt = static_cast<float*>(scratch);
+    unsigned char* live = reinterpret_cast<unsigned char*>(mt + items * kRowRun);
+    ra.mt = mt; ra.live = live;
+    if (blocks > 1 && !accumulate)
+        KTM_CUDA_TRY(cudaMemsetAsync(data, 0, (size_t)pitch * sizeof(float) * g.ntr, s));
+    row_model_kernel<<<(unsigned)((items + 7) / 8), 256, 0, s>>>(a, ra.nruns, mt, live);
+    KTM_CUDA_TRY(cudaGetLastError());
+    const dim3 grid((unsigned)groups, (unsigned)blocks);
+    return wt == 2 ? launch_rows<2>(ra, grid, smem, s)
+         : wt == 1 ? launch_rows<1>(ra, grid, smem, s) : launch_rows<0>(ra, grid, smem, s);
+}
+
 }  // namespace
 
 int launch_demigrate(const Geometry& g, const float* midX, const float* midY, const float* offX,
                      const float* offY, const float* vel, int velCube, const float* image,
                      float* data, int pitch, int pick, int weightMethod, float aperture,
-                     int accumulate, cudaStream_t s)
+                     int accumulate, void* scratch, cudaStream_t s)
 {
     if (pitch < g.nt + 2 || pitch % 4 != 0)
         return set_error(KTM_ERR_ARG, "demigrate: dataPitch must be >= tracePts + 2 and a multiple of 4");
     const size_t pitchBytes = (size_t)pitch * sizeof(float);
+    const bool empty = g.ntr == 0 || (long long)g.nx * g.ny * g.nz == 0;
+    int dev = 0, sm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
+    const size_t need = empty ? 0 : demigrate_scratch(g, velCube, pick, weightMethod);
+    void* own = nullptr;
+    if (need && !scratch && pool_malloc(&own, need, s) != cudaSuccess) {
+        cudaGetLastError();              // no room for the copy of the model: the shared rows
+        own = nullptr;
+    }
+    if (need && (scratch || own)) {
+        const int rc = launch_row_demigrate(g, midX, midY, offX, offY, vel, image, data, pitch, weightMethod, aperture,
+                                            accumulate, scratch ? scratch : own, sm, s);
+        if (own) cudaFreeAsync(own, s);
+        return rc;
+    }
     if (!accumulate && g.ntr > 0)
         KTM_CUDA_TRY(cudaMemsetAsync(data, 0, pitchBytes * g.ntr, s));
-    if (g.ntr == 0 || (long long)g.nx * g.ny * g.nz == 0) return KTM_OK;
+    if (empty) return KTM_OK;
     const int wt = weightMethod == KTM_WEIGHT_SQRT ? 1 : weightMethod == KTM_WEIGHT_PREFOLD ? 2 : 0;
     // the sqrt(j dt) table only for the table weight; the coordinates' alignment pad
     const size_t fixed = (wt == 0 ? (size_t)padded_pitch(g.nt + 1) * sizeof(float2) : 0) + 64;
@@ -296,9 +659,6 @@ int launch_demigrate(const Geometry& g, const float* midX, const float* midY, co
         return set_error(KTM_ERR_LIMIT, "demigrate: tracePts=%d exceeds the shared-memory limit", g.nt);
     const size_t smem = fixed + chunk * perTrace;
 
-    int dev = 0, sm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
     const int ncols = g.nx * g.ny;
     const int chunks = (g.ntr + chunk - 1) / chunk;
     // column blocks only when the traces alone give too few CTAs (then the

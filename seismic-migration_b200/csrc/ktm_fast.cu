@@ -533,8 +533,9 @@ Stages fast_stages(const FastArgs& a, int esize, bool table)
 
 // Trace slices of a launch of `base` CTAs per slice on `slots` resident CTAs: the number
 // with the least estimated time, in traces of a CTA: a CTA takes its traces + 8 for its
-// prologue; up to `slots` of them run at once, more end unevenly (aperture, trace end), half a
-// CTA past the mean; plus the partial images (a trace takes about 1 us at R = 16, 6.5 MB of
+// prologue, and the last ones end half a CTA past the mean (columns keep uneven numbers of
+// traces: 168 x 206 image, 8232 traces without aperture, 39 us in 64 slices, 54 in the 21 that
+// fit at once); plus the partial images (a trace takes about 1 us at R = 16, 6.5 MB of
 // partial images the same).
 int choose_slices(long long base, int slots, int ntr, int R, size_t nimg, int most)
 {
@@ -542,7 +543,7 @@ int choose_slices(long long base, int slots, int ntr, int R, size_t nimg, int mo
     float least = 3.0e38f;
     for (int s = 1; s <= most; s++) {
         const float per = (float)((ntr + s - 1) / s) + 8.0f;
-        const float rounds = base * s <= slots ? 1.0f : (float)(base * s) / (float)slots + 0.5f;
+        const float rounds = std::max(1.0f, (float)(base * s) / (float)slots) + 0.5f;
         const float copies = s > 1 ? (float)s * (float)nimg * (8.0f / 6.5e6f) * 16.0f / (float)R : 0.0f;
         const float cost = rounds * per + copies;
         if (cost < least) {

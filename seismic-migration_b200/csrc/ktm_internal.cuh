@@ -82,11 +82,14 @@ int take_wait_stalls(cudaStream_t s, bool deviceSync, unsigned* n);
 // a barrier nothing arrives on); checksum = sum of the 64 KiB of 0x01 bytes landed.
 int wait_selftest(int stall, unsigned long long limitNs, unsigned* checksum);
 
-// ktm_adjoint.cu: demigration into the packed F32 layout [ntr][pitch]
+// ktm_adjoint.cu: demigration into the packed F32 layout [ntr][pitch].  demigrate_scratch:
+// device bytes of the model copy a job's kernel reads (0: none); launch_demigrate allocates
+// them stream-ordered where scratch is NULL.
+size_t demigrate_scratch(const Geometry& g, int velCube, int pick, int weightMethod);
 int launch_demigrate(const Geometry& g, const float* midX, const float* midY, const float* offX,
                      const float* offY, const float* vel, int velCube, const float* image,
                      float* data, int pitch, int pick, int weightMethod, float aperture,
-                     int accumulate, cudaStream_t s);
+                     int accumulate, void* scratch, cudaStream_t s);
 
 // ktm_api.cu: stream-ordered temporary allocations from the library's own memory
 // pool on the current device (release threshold unlimited, so repeated calls
