@@ -1062,6 +1062,12 @@ int take_wait_stalls(cudaStream_t s, bool deviceSync, unsigned* n)
     return KTM_OK;
 }
 
+int copy_wait_stalls(void* dst, cudaStream_t s)
+{
+    KTM_CUDA_TRY(cudaMemcpyFromSymbolAsync(dst, g_waitStalls, sizeof(unsigned), 0, cudaMemcpyDeviceToDevice, s));
+    return KTM_OK;
+}
+
 int wait_selftest(int stall, unsigned long long limitNs, unsigned* checksum)
 {
     constexpr unsigned kBytes = 64 * 1024, kWords = kBytes / 4;

@@ -78,6 +78,8 @@ int launch_batch(const FastArgs* jobs, int njobs, cudaStream_t s);
 // bulk copy ran out (the count is reset when read).  Read on stream s after the
 // caller's work on s; deviceSync: after all work on the device.
 int take_wait_stalls(cudaStream_t s, bool deviceSync, unsigned* n);
+// The count into device memory (4 bytes) on stream s, without a reset.
+int copy_wait_stalls(void* dst, cudaStream_t s);
 // One-CTA self-test of the bulk copy and its bounded wait (stall: wait first on
 // a barrier nothing arrives on); checksum = sum of the 64 KiB of 0x01 bytes landed.
 int wait_selftest(int stall, unsigned long long limitNs, unsigned* checksum);
