@@ -196,7 +196,11 @@ __global__ void __launch_bounds__(FftShape<LOGM, FILTER>::kThreads, FftShape<LOG
     using S = FftShape<LOGM, FILTER>;
     constexpr int M = S::M, E = S::E, T = S::T, R = S::kLast, G = E / R, P = S::kPasses;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ float2 red[S::kThreads / 32 + 1];
+    // the warps' maxima: two sets in turn where the barrier before they are read is the only
+    // one of a round, so that a warp in the next round writes none that is still to be read;
+    // the transform's barriers keep the rounds apart
+    __shared__ float2 red[FILTER ? 1 : 2][S::kThreads / 32 + 1];
+    int set = 0;
     const int t = threadIdx.x % T, sub = threadIdx.x / T;
     float2* zs = reinterpret_cast<float2*>(smem_raw) + (size_t)sub * M;
     // z of each pair, twiddles, |H| [E][T], fold weights [M]
@@ -358,14 +362,15 @@ __global__ void __launch_bounds__(FftShape<LOGM, FILTER>::kThreads, FftShape<LOG
                 my = fmaxf(my, __shfl_xor_sync(0xffffffffu, my, o));
             }
             if (T > 32) {
-                if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_float2(mx, my);
+                if ((threadIdx.x & 31) == 0) red[set][threadIdx.x >> 5] = make_float2(mx, my);
                 __syncthreads();
 #pragma unroll 8
                 for (int w = 0; w < T / 32; w++) {
-                    const float2 o = red[sub * (T / 32) + w];
+                    const float2 o = red[set][sub * (T / 32) + w];
                     mx = fmaxf(mx, o.x);
                     my = fmaxf(my, o.y);
                 }
+                if constexpr (!FILTER) set ^= 1;
             }
         }
         const float sx = trace_scale(a.fmt, mx), sy = trace_scale(a.fmt, my);

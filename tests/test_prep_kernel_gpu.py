@@ -111,3 +111,23 @@ def test_script_order_of_odd_counts(cuda, ktm_lib):
     for opt in (0, 3):
         a, b = (_prepare(x, 0.002, opt, script_order=o).data for o in (False, True))
         assert torch.equal(torch.roll(a, -1, 0), b)
+
+
+@pytest.mark.parametrize("fmt", ["f16", "bf16"])
+@pytest.mark.parametrize("ntr,nt", [(24001, 601), (16001, 1001), (12001, 1501), (6001, 4096),
+                                    (3001, 6001), (2001, 16384)])
+def test_many_rounds_without_a_filter(cuda, ktm_lib, ntr, nt, fmt):
+    """Counts that give every CTA several rounds, neighbouring traces whose maxima differ by
+    orders of magnitude: each trace keeps its own scale, every sample is quantised by it."""
+    import torch
+    gen = torch.Generator(device=cuda)
+    gen.manual_seed(nt)
+    x = torch.randn((ntr, nt), device=cuda, generator=gen)
+    x *= torch.pow(2.0, torch.randint(-20, 21, (ntr, 1), device=cuda, generator=gen).float())
+    x[:, 0] = 0
+    top = x.abs().amax(1) / (32768.0 if fmt == "f16" else 1.0)
+    want = (x * (1.0 / top)[:, None]).to(torch.float16 if fmt == "f16" else torch.bfloat16)
+    for _ in range(5):
+        p = _prepare(x, 0.002, 0, fmt=fmt)
+        assert torch.equal(p.scale, top)
+        assert torch.equal(p.data[:, :nt], want) and not p.data[:, nt:].any()
