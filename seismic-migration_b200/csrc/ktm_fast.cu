@@ -532,21 +532,35 @@ Stages fast_stages(const FastArgs& a, int esize, bool table)
     return s;
 }
 
-// Trace slices of a launch of `base` CTAs per slice on `slots` resident CTAs: the number
-// with the least estimated time, in traces of a CTA: a CTA takes its traces + 8 for its
-// prologue, and the last ones end half a CTA past the mean (columns keep uneven numbers of
-// traces: 168 x 206 image, 8232 traces without aperture, 39 us in 64 slices, 54 in the 21 that
-// fit at once); plus the partial images (a trace takes about 1 us at R = 16, 6.5 MB of
-// partial images the same).
-int choose_slices(long long base, int slots, int ntr, int R, size_t nimg, int most)
+// Partial images of a launch at most: an image of more than half of this is written in place.
+constexpr size_t kPartialBytes = 64u << 20;
+
+// Trace slices of a launch of `base` CTAs per slice on `slots` resident CTAs: the number with
+// the least estimated time in microseconds.  A CTA takes R / 16 for a trace, times the share of
+// the image that an aperture covers, and 2 + 6 R / 16 for its prologue, first copy and write-out.
+// Columns keep uneven numbers of traces, so that the longest CTA of a single round takes 1.3 of
+// the mean, two rounds 2.4, and more end half a round past it.  Partial images are written and
+// read once, and one more kernel (4) sums them.
+// Fitted to 112 launches (1 to 22,500 columns, 33 to 1501 samples, 100 to 60,000 traces), each
+// in 1 to 64 slices: the choice is on average 2 % off the best of them.  128 x 751 image, 6144
+// traces without aperture: 443 us in the 11 slices that fit at once, 354 in 64; 256 x 1001,
+// 1500 traces with an aperture of 700 m: 88 us in 6, 146 in 64.
+int choose_slices(const FastArgs& a, long long base, int slots, int R)
 {
+    const Geometry& g = a.g;
+    const size_t nimg = (size_t)g.nx * g.ny * g.nz;
+    const int most = (int)std::min<size_t>(std::max(1, std::min(64, g.ntr / 4)),
+                                           std::max<size_t>(1, kPartialBytes / (nimg * sizeof(float))));
+    auto covered = [&](float extent) { return std::min(1.0f, 2.0f * a.aperture / std::max(fabsf(extent), 1e-30f)); };
+    const float share = a.aperture > 0.0f ? std::max(0.1f, covered((float)g.nx * g.dx) * covered((float)g.ny * g.dy)) : 1.0f;
+    const float run = (float)R / 16.0f;
     int best = 1;
     float least = 3.0e38f;
     for (int s = 1; s <= most; s++) {
-        const float per = (float)((ntr + s - 1) / s) + 8.0f;
-        const float rounds = std::max(1.0f, (float)(base * s) / (float)slots) + 0.5f;
-        const float copies = s > 1 ? (float)s * (float)nimg * (8.0f / 6.5e6f) * 16.0f / (float)R : 0.0f;
-        const float cost = rounds * per + copies;
+        const float per = (float)((g.ntr + s - 1) / s) * run * share + 2.0f + 6.0f * run;
+        const float r = (float)(base * s) / (float)slots;
+        const float rounds = r <= 1.0f ? 1.3f : r <= 2.0f ? 2.4f : r + 0.5f;
+        const float cost = rounds * per + (s > 1 ? (float)s * (float)nimg * (8.0f / 6.5e6f) + 4.0f : 0.0f);
         if (cost < least) {
             least = cost;
             best = s;
@@ -576,11 +590,9 @@ int launch_block(const FastArgs& a, cudaStream_t stream, int smCount)
     const unsigned gy = (unsigned)((g.nz + 32 * R - 1) / (32 * R));
     if (gy > 65535) return set_error(KTM_ERR_LIMIT, "fast kernel: Nz too large");
     const size_t nimg = (size_t)cols * g.nz;
-    // at least eight traces to a slice, at most 64 slices
     int slices = a.slices > 0 ? min(a.slices, max(1, g.ntr))
-                              : choose_slices((long long)gx * gy, SH::kMinBlocks * smCount, g.ntr, R, nimg,
-                                              max(1, min(64, g.ntr / 8)));
-    const int perSlice = (g.ntr + slices - 1) / slices;
+                              : choose_slices(a, (long long)gx * gy, SH::kMinBlocks * smCount, R);
+    int perSlice = (g.ntr + slices - 1) / slices;
     slices = (g.ntr + perSlice - 1) / perSlice;
 
     float* partial = nullptr;
@@ -588,8 +600,15 @@ int launch_block(const FastArgs& a, cudaStream_t stream, int smCount)
         if (a.scratch && a.scratchBytes >= (size_t)slices * nimg * sizeof(float)) {
             partial = static_cast<float*>(a.scratch);
         } else {
-            KTM_CUDA_TRY(pool_malloc(reinterpret_cast<void**>(&partial),
-                                         (size_t)slices * nimg * sizeof(float), stream));
+            const cudaError_t m = pool_malloc(reinterpret_cast<void**>(&partial),
+                                              (size_t)slices * nimg * sizeof(float), stream);
+            if (m != cudaSuccess && a.slices > 0) KTM_CUDA_TRY(m);
+            if (m != cudaSuccess) {
+                cudaGetLastError();            // no room for partial images: one slice, in place
+                partial = nullptr;
+                slices = 1;
+                perSlice = g.ntr;
+            }
         }
     }
     dim3 grid(gx, gy, (unsigned)slices);
