@@ -105,6 +105,8 @@ struct ChunkSync {
 };
 static_assert(sizeof(ChunkSync) + sizeof(FastArgs) + sizeof(int) <= 1024,
               "static shared memory of the fast kernels within the 1 KB allowance");
+// the 227 KB of a CTA hold its static shared memory too
+constexpr size_t kMaxDynamic = kMaxSmemBytes - 1024;
 
 // Traces per row buffer and row buffers of a launch.
 struct Stages {
@@ -528,7 +530,7 @@ Stages fast_stages(const FastArgs& a, int esize, bool table)
     Stages s = fit(3);
     if (s.chunk < std::min(cap, 16)) s = fit(2);
     // the longest traces: two buffers leave no room for the warps' tables
-    if (chunk_layout(s, SH::kWarps, a.pitch, esize, a.g.nt, table).total > (size_t)kMaxSmemBytes) s.stages = 1;
+    if (chunk_layout(s, SH::kWarps, a.pitch, esize, a.g.nt, table).total > kMaxDynamic) s.stages = 1;
     return s;
 }
 

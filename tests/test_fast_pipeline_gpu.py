@@ -76,3 +76,29 @@ def test_one_buffer(cuda, ktm_lib):
     assert np.linalg.norm(got - want) <= REL * longest / 700.0 * np.linalg.norm(want)
     with pytest.raises(ktm.KtmError):
         _run(cuda, _case(3, 2, longest + 4, 2, 30, 0.05), "table")
+
+
+@pytest.mark.parametrize("batch", [False, True])
+@pytest.mark.parametrize("fmt,weight,lo,hi", [("f32", "prefold", 28774, 28818), ("f32", "sqrt", 28774, 28818),
+                                              ("f32", "table", 14386, 14410), ("f16", "table", 19182, 19212),
+                                              ("bf16", "table", 19182, 19212)])
+def test_every_length_around_the_last_two_buffers(cuda, ktm_lib, fmt, weight, lo, hi, batch):
+    """From two buffers beside the warps' tables to one, every trace length on the way."""
+    import torch
+
+    import ktm
+    rel = {"f32": 0.0, "f16": 6e-4, "bf16": 4e-3}[fmt]             # storage: half an ulp of the largest sample
+    for nt in range(lo, hi, 1 if not batch else 2):
+        case = _case(nt, 3, nt, 2, 40, 0.3)
+        g, mx, my, ox, oy, tr, vel = case
+        want = oracle.migrate_f64(*g, 0.004, mx, my, ox, oy, tr, vel, pick=1,
+                                  prefold={"prefold": 1, "table": 0, "sqrt": 0}[weight], aperture=0.0)
+        if batch:
+            t = [torch.as_tensor(a).to(cuda) for a in (mx, my, ox, oy, vel, tr)]
+            packed = ktm.prepare(t[5], 0.004, fmt=fmt, rho=0, prefold=weight == "prefold")
+            job = dict(imageX=g[0], imageY=g[1], imageZ=g[2], dt=0.004, midX=t[0], midY=t[1], offX=t[2], offY=t[3],
+                       velocity=t[4], traces=packed, weight=weight, image=torch.empty(want.shape, device=cuda))
+            got = ktm.migrate_batch([job])[0].cpu().numpy()
+        else:
+            got = _run(cuda, case, weight, fmt)
+        assert np.linalg.norm(got - want) <= (REL * nt / 700.0 + rel) * np.linalg.norm(want), nt
