@@ -472,6 +472,8 @@ RefSplit ref_split(const Geometry& g, int R, int sm)
         const int cap = r == 4 ? RefShape<4>::kWarpsPerSm : RefShape<1>::kWarpsPerSm;
         const long long runs = (g.nz + 32LL * r - 1) / (32 * r);
         for (int w = 1; w <= cap && w <= cols; w++) {
+            // two stages of one trace and the warps' tables must fit a CTA (one warp's always do)
+            if (w > 1 && ref_smem(1, g.stride, g.nt, w).total > (size_t)kMaxSmemBytes) break;
             const long long ctas = (cols + w - 1) / w * runs, load = (ctas + sm - 1) / sm;
             // CTAs of an SM at a time, by registers and by two stages of a trace each
             int perSm = (int)std::min<long long>(cap / w, load);

@@ -103,3 +103,12 @@ def test_special_samples_at_zero_tau_and_accumulation(cuda, ktm_lib):
     start[0, 0, :3] = -0.0
     with np.errstate(invalid="ignore"):
         assert same_with_nans(_run(cuda, case, start=start.copy()), start + ref)
+
+
+@pytest.mark.parametrize("run", [0, 32, 64])
+@pytest.mark.parametrize("nt,nx,ny,nz", [(28856, 40, 1, 40), (28900, 80, 50, 64), (28924, 74, 64, 64), (28924, 60, 50, 1),
+                                         (28900, 25, 1, 129), (28880, 500, 2, 33)])
+def test_longest_traces_of_wide_images(cuda, ktm_lib, nt, nx, ny, nz, run):
+    """The longest accepted traces leave room for fewer warps' tables than an SM has warps."""
+    case = _case(nt + nx, 2, nt, nx, ny, nz, dt=0.001)
+    assert same_with_nans(_run(cuda, case, run=run), _oracle(case))
