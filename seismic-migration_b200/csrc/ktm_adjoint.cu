@@ -625,7 +625,7 @@ int launch_row_demigrate(const Geometry& g, const float* midX, const float* midY
 int launch_demigrate(const Geometry& g, const float* midX, const float* midY, const float* offX,
                      const float* offY, const float* vel, int velCube, const float* image,
                      float* data, int pitch, int pick, int weightMethod, float aperture,
-                     int accumulate, void* scratch, cudaStream_t s)
+                     int accumulate, void* scratch, bool mayAllocate, cudaStream_t s)
 {
     if (pitch < g.nt + 2 || pitch % 4 != 0)
         return set_error(KTM_ERR_ARG, "demigrate: dataPitch must be >= tracePts + 2 and a multiple of 4");
@@ -636,7 +636,7 @@ int launch_demigrate(const Geometry& g, const float* midX, const float* midY, co
     cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
     const size_t need = empty ? 0 : demigrate_scratch(g, velCube, pick, weightMethod);
     void* own = nullptr;
-    if (need && !scratch && pool_malloc(&own, need, s) != cudaSuccess) {
+    if (need && !scratch && mayAllocate && pool_malloc(&own, need, s) != cudaSuccess) {
         cudaGetLastError();              // no room for the copy of the model: the shared rows
         own = nullptr;
     }

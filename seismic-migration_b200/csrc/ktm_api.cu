@@ -559,7 +559,7 @@ extern "C" int ktmDemigrate(const ktm_job* job, float* data, int dataPitch)
         return set_error(KTM_ERR_ARG, "NULL model or velocity");
     rc = launch_demigrate(g, job->midX, job->midY, job->offX, job->offY, job->velocity,
                           job->velocityCube, job->image, data, dataPitch, job->pick,
-                          job->weightMethod, job->aperture, job->accumulate, nullptr,
+                          job->weightMethod, job->aperture, job->accumulate, nullptr, true,
                           static_cast<cudaStream_t>(job->stream));
     return rc ? rc : set_ok();
 }

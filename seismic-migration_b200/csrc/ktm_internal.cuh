@@ -85,13 +85,14 @@ int copy_wait_stalls(void* dst, cudaStream_t s);
 int wait_selftest(int stall, unsigned long long limitNs, unsigned* checksum);
 
 // ktm_adjoint.cu: demigration into the packed F32 layout [ntr][pitch].  demigrate_scratch:
-// device bytes of the model copy a job's kernel reads (0: none); launch_demigrate allocates
-// them stream-ordered where scratch is NULL.
+// device bytes of the model copy a job's kernel reads (0: none).  launch_demigrate takes them
+// from scratch, or allocates them stream-ordered where that is NULL and mayAllocate is set; without
+// them it runs the kernel that needs none.
 size_t demigrate_scratch(const Geometry& g, int velCube, int pick, int weightMethod);
 int launch_demigrate(const Geometry& g, const float* midX, const float* midY, const float* offX,
                      const float* offY, const float* vel, int velCube, const float* image,
                      float* data, int pitch, int pick, int weightMethod, float aperture,
-                     int accumulate, void* scratch, cudaStream_t s);
+                     int accumulate, void* scratch, bool mayAllocate, cudaStream_t s);
 
 // ktm_api.cu: stream-ordered temporary allocations from the library's own memory
 // pool on the current device (release threshold unlimited, so repeated calls

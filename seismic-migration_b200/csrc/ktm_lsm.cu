@@ -130,7 +130,7 @@ struct Lsm {
     float *r, *q, *s, *p, *ones;
     float* rw;                  // prefolded weight: the folded residual the migration reads
     void* scratch; size_t scratchBytes; int slices;
-    void* demig;                // the demigration's copy of the model (NULL: it needs none)
+    void* demig;                // the demigration's copy of the model (NULL: it needs none, or there is no room)
     double *partial, *sc, *rnorm, *gnorm;
     cudaStream_t st;
 
@@ -168,7 +168,7 @@ struct Lsm {
     {
         return launch_demigrate(g, job->midX, job->midY, job->offX, job->offY, job->velocity,
                                 job->velocityCube, image, data, pitch, job->pick, job->weightMethod,
-                                job->aperture, 0, demig, st);
+                                job->aperture, 0, demig, false, st);
     }
     unsigned blocks(size_t n) const
     {
@@ -242,14 +242,20 @@ extern "C" int ktmLeastSquaresMigrate(const ktm_lsm* L)
     s.slices = (int)std::min<size_t>(64, std::max<size_t>(1, (size_t(256) << 20) / (s.nm * 4)));
     s.scratchBytes = (size_t)s.slices * s.nm * sizeof(float);
     const bool fold = j->weightMethod == KTM_WEIGHT_PREFOLD;
-    const size_t demigBytes = demigrate_scratch(s.g, j->velocityCube, j->pick, j->weightMethod);
+    size_t demigBytes = demigrate_scratch(s.g, j->velocityCube, j->pick, j->weightMethod);
     // every piece starts on a 256-byte boundary (take() below)
     auto r256 = [](size_t n) { return (n + 255) / 256 * 256; };
-    const size_t bytes = r256(kDotBlocks * sizeof(double)) + r256(kNScalars * sizeof(double)) +
+    size_t bytes = r256(kDotBlocks * sizeof(double)) + r256(kNScalars * sizeof(double)) +
                          2 * r256((its + 1) * sizeof(double)) + (fold ? 3 : 2) * r256(s.nd * 4) +
                          2 * r256(s.nm * 4) + r256((size_t)s.g.ntr * 4) + r256(s.scratchBytes) + r256(demigBytes);
     unsigned char* ws = nullptr;
     cudaError_t e = pool_malloc(reinterpret_cast<void**>(&ws), bytes, s.st);
+    if (e != cudaSuccess && demigBytes) {
+        cudaGetLastError();              // no room for the copy of the model: the kernel without it
+        bytes -= r256(demigBytes);
+        demigBytes = 0;
+        e = pool_malloc(reinterpret_cast<void**>(&ws), bytes, s.st);
+    }
     if (e != cudaSuccess) {
         if (ownStream) cudaStreamDestroy(s.st);
         return set_error(KTM_ERR_NOMEM, "ktmLeastSquaresMigrate: workspace of %zu bytes: %s", bytes,
