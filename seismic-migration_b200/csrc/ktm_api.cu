@@ -69,7 +69,9 @@ cudaError_t pool_malloc(void** p, size_t bytes, cudaStream_t s)
         }
         pool = g_pool[dev];
     }
-    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+    e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();   // reported here, not by the next launch's check
+    return e;
 }
 
 namespace {

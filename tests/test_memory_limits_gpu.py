@@ -1,5 +1,5 @@
-"""Least squares where the demigration's copy of the model finds no room on the device: the
-solver runs the demigration that needs none."""
+"""Calls that find little room on the device: least squares without the demigration's copy of the
+model, and a failed allocation that leaves the next call alone."""
 from __future__ import annotations
 
 import numpy as np
@@ -48,3 +48,39 @@ def test_without_room_for_the_model_copy(cuda, ktm_lib, graph):
     np.testing.assert_allclose(r, residuals, rtol=1e-5)
     np.testing.assert_allclose(q, gradients, rtol=1e-4)
     assert float((model.double() - want.double()).norm() / want.double().norm()) <= 1e-4
+
+
+def test_a_failed_allocation_stays_in_its_call(cuda, ktm_lib):
+    """A call that finds no memory reports it; the next one runs."""
+    import torch
+
+    import ktm
+    from ktm import inverse
+    nx, nz, ntr, nt = 300000, 64, 40, 100
+    zero = torch.zeros(ntr, device=cuda)
+    wide, narrow = (inverse.MigrationOperator(imageX=(n, 0.5, 0.0), imageY=(1, 1.0, 0.0), imageZ=(nz, 0.002, 0.0), dt=0.004,
+                                              nt=nt, midX=zero, midY=zero, offX=zero, offY=zero, aperture=100.0,
+                                              velocity=torch.full((nz,), 2000.0, device=cuda), weight="prefold")
+                    for n in (nx, 50))
+    model, image = torch.zeros((nx, 1, nz), device=cuda), torch.ones((50, 1, nz), device=cuda)
+    data = wide.pack(torch.ones((ntr, nt), device=cuda))
+    out = torch.empty_like(data)
+    want = narrow.demigrate(image).clone()
+    torch.cuda.synchronize()
+    ktm._lib.check(ktm_lib.ktmReleaseMemory())
+    torch.cuda.empty_cache()
+    taken, size = [], 1 << 34
+    try:
+        while size >= 32 * MB:
+            try:
+                taken.append(torch.empty(size, dtype=torch.uint8, device=cuda))
+            except torch.cuda.OutOfMemoryError:
+                size //= 2
+        with pytest.raises(ktm.KtmError):
+            wide.least_squares(data, 1, model=model)       # some 400 MB
+    finally:
+        taken.clear()
+        torch.cuda.empty_cache()
+    narrow.demigrate(image, out)
+    # two column blocks added in either order
+    assert torch.allclose(out, want, rtol=1e-5, atol=1e-5 * float(want.abs().max()))
