@@ -941,11 +941,8 @@ def main():
                          "sfu_issued": {"achieved_tsqrt_s": sfu_rate / 1e12,
                                         "peak_tsqrt_s": sq.value / 1e12,
                                         "frac": sfu_rate / sq.value,
-                                        "note": ("2 sqrt.approx per counted pair, sqrt(t) prefolded "
-                                                 "into the samples; a trace that ends within a run "
-                                                 "is counted for the run and walked to its last "
-                                                 "step only, so fewer are issued"
-                                                 if a.weight == "prefold" else
+                                        "note": ("2 sqrt.approx per pair, sqrt(t) prefolded into "
+                                                 "the samples" if a.weight == "prefold" else
                                                  "2 sqrt.approx per pair, plus the weight's "
                                                  "table lookup or third sqrt.approx")},
                          "traffic_note": MIGRATE_DRAM_NOTE,

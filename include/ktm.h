@@ -160,7 +160,10 @@ typedef struct ktm_job {
                                                   linear pick with the prefolded or table
                                                   weight.  ktmAutotuneTile chooses these. */
     unsigned long long* pairsEvaluated;        /* optional device counter: pairs the
-                                                  kernel evaluated (after culling) */
+                                                  kernel evaluated (after culling; of a
+                                                  trace that ends within a tau run, with
+                                                  prefolded samples, up to its last step of
+                                                  64 samples) */
     /* FAST mode with raw (not packed) traces: the library prepares them first */
     int   rho;                                 /* KTM_RHO_* pre-filter (ktmApplyRhoFilter.m) */
     int   packFormat;                          /* KTM_FMT_* of the packed samples */
@@ -294,7 +297,7 @@ int ktmLeastSquaresMigrate(const ktm_lsm* lsm);
 /* ------------------------------------------------------------------------ */
 
 /* Many independent jobs (image patches of any size, trace sets of any size) in
- * ONE persistent launch: a queue of (job, 8 image columns, tau run, trace slice)
+ * ONE persistent launch: a queue of (job, image columns, tau run, trace slice)
  * tiles sorted longest first, pulled by one CTA per SM slot.  Every job: FAST
  * mode, device memory, a packed trace set; all jobs share the trace format,
  * pick and weight, and the first job's tileRun (0: chosen from the jobs' Nz).

@@ -244,7 +244,7 @@ __device__ __forceinline__ bool fast_tile(const FastArgs& a, Stages st, int colG
     const float upast2 = (umax * 1.0001f + 1.0f) * (umax * 1.0001f + 1.0f);
     const float ap2 = a.aperture > 0.0f ? a.aperture * a.aperture : -1.0f;
     const f2 M2 = pk(kMagic, kMagic);
-    unsigned keptTraces = 0;        // traces this warp evaluated (all lanes agree)
+    unsigned walked = 0;            // pairs evaluated of the traces this lane looked at
 
     if (threadIdx.x == 0) {
         for (int b = 0; b < st.stages; b++) {
@@ -283,6 +283,7 @@ __device__ __forceinline__ bool fast_tile(const FastArgs& a, Stages st, int colG
 #pragma unroll
                 for (int d = H > 4 ? 4 : 2; kStepwise && d > 0; d >>= 1)
                     if (hmax - 1 + d < H && reaches(hmax - 1 + d)) hmax += d;
+                walked += (unsigned)(kStepwise ? min(64 * hmax, nvalid) : nvalid);
             }
         }
         const unsigned kept = __ballot_sync(0xffffffffu, hmax > 0);
@@ -297,7 +298,6 @@ __device__ __forceinline__ bool fast_tile(const FastArgs& a, Stages st, int colG
             tab[__popc(kept & ((1u << lane) - 1u))] = make_float4(ds, dr, sc, __uint_as_float(row + (unsigned)hmax));
         }
         __syncwarp();
-        keptTraces += (unsigned)cnt;
         // the ch/stages-th use of buffer b completes that phase of its barrier
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(&cs.bar[b], (unsigned)parity, kBulkWaitNs))) {
             if (lane == 0) {
@@ -440,8 +440,10 @@ __device__ __forceinline__ bool fast_tile(const FastArgs& a, Stages st, int colG
             }
         }
     }
-    if (a.pairsEvaluated && lane == 0 && keptTraces)
-        atomicAdd(a.pairsEvaluated, (unsigned long long)keptTraces * (unsigned long long)nvalid);
+    if (a.pairsEvaluated && colValid) {
+        const unsigned lo = __reduce_add_sync(0xffffffffu, walked & 0xffffu), hi = __reduce_add_sync(0xffffffffu, walked >> 16);
+        if (lane == 0 && (lo | hi)) atomicAdd(a.pairsEvaluated, ((unsigned long long)hi << 16) + lo);
+    }
     return true;
 }
 

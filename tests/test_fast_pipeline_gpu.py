@@ -102,3 +102,34 @@ def test_every_length_around_the_last_two_buffers(cuda, ktm_lib, fmt, weight, lo
         else:
             got = _run(cuda, case, weight, fmt)
         assert np.linalg.norm(got - want) <= (REL * nt / 700.0 + rel) * np.linalg.norm(want), nt
+
+
+@pytest.mark.parametrize("weight,pick", [("prefold", "linear"), ("table", "linear"), ("sqrt", "truncate")])
+@pytest.mark.parametrize("run", [256, 384, 512])
+@pytest.mark.parametrize("ntr,nt,nx,nz,aperture", [(50, 300, 7, 700, 0.0), (333, 260, 30, 515, 400.0), (1, 90, 1, 64, 0.0)])
+def test_counts_the_pairs_it_evaluates(cuda, ktm_lib, ntr, nt, nx, nz, aperture, run, weight, pick):
+    """Prefolded samples: each kept trace up to the last 64-sample step that starts before its end;
+    the other weights: the whole run.  The kernel's bound lies 1e-4 and a sample past the end."""
+    import torch
+    g, mx, my, ox, oy, tr, vel = _case(ntr + nz, ntr, nt, nx, nz, 0.002)
+    vel[:] = 2000.0
+    counter = torch.zeros(1, dtype=torch.int64, device=cuda)
+    _run(cuda, (g, mx, my, ox, oy, tr, vel), weight, "f32", pick=pick, aperture=aperture, tile_run=run, pairs_counter=counter)
+    x = np.float64(g[0].imageStart) + np.float64(g[0].imageStep) * np.arange(nx)
+    tau = np.float64(np.float32(0.002)) * np.arange(nz)
+    bounds = []
+    for sign in (-1.0, 1.0):
+        total = 0
+        for c in range(nx):
+            d = mx.astype(np.float64) - x[c]
+            ok = np.abs(d) <= aperture * (1.0 + sign * 1e-6) if aperture else np.full(ntr, True)
+            u = sum(np.sqrt(tau ** 2 + ((d + s * ox)[:, None] / 2000.0) ** 2) for s in (-1.0, 1.0)) / np.float64(np.float32(0.004))
+            early = u < (nt * 1.0001 + 1.0) * (1.0 + sign * 1e-5)
+            for r0 in range(0, nz, run):
+                valid = min(run, nz - r0)
+                steps = early[:, r0:r0 + run:64].sum(1)
+                per = np.minimum(64 * steps, valid) if weight == "prefold" else np.where(steps > 0, valid, 0)
+                total += int(per[ok].sum())
+        bounds.append(total)
+    assert bounds[0] <= int(counter[0]) <= bounds[1], (bounds, int(counter[0]))
+    assert bounds[1] - bounds[0] <= 0.02 * bounds[1] + 512
