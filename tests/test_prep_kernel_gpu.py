@@ -131,3 +131,26 @@ def test_many_rounds_without_a_filter(cuda, ktm_lib, ntr, nt, fmt):
         p = _prepare(x, 0.002, 0, fmt=fmt)
         assert torch.equal(p.scale, top)
         assert torch.equal(p.data[:, :nt], want) and not p.data[:, nt:].any()
+
+
+@pytest.mark.parametrize("opt", [1, 2, 3])
+@pytest.mark.parametrize("nt", [2, 4, 8])
+def test_the_filter_is_rounded_once(cuda, ktm_lib, nt, opt):
+    """One line of the spectrum, whose transform is exact: the result is the filter's own value,
+    |w|, sqrt(|w| / 2) or w at a quarter of the sampling rate (at half of it for two samples), in
+    64 bits rounded to FP32."""
+    import torch
+    rng = np.random.default_rng(nt)
+    for dt in np.exp(rng.uniform(np.log(2e-4), np.log(2e-2), 200)).astype(np.float32):
+        n = np.arange(nt)
+        x = np.where(n % 2 == 0, 1.0, -1.0) if nt == 2 else np.rint(np.cos(np.pi * n / 2))
+        got = _prepare(torch.as_tensor(x[None].astype(np.float32)).to(cuda), float(dt), opt).unpacked()[0].cpu().numpy()
+        w = 2.0 * np.pi * (nt // 4 if nt > 2 else 1) / np.float64(dt)
+        size = np.float32([0, w, np.sqrt(w / 2.0), w][opt])
+        if nt == 2:                                     # Nyquist: the real part alone
+            want = [0.0, 0.0 if opt == 3 else -size]
+        else:
+            c, s = np.rint(np.cos(np.pi * n / 2)), np.rint(np.sin(np.pi * n / 2))
+            want = size * [0, c, c - s, -s][opt]
+            want[0] = 0.0
+        assert np.array_equal(got, np.float32(want)), (dt, got, want)
