@@ -171,18 +171,18 @@ struct FftShape {
     // 16 warps of 128 registers per SM with the transform (where a CTA is not larger): 20 warps
     // of 96 take 300 us instead of 297 for 62,500 traces of 1501 samples; 32 warps without it
     static constexpr int kCtasPerSm = kThreads >= 1024 ? 1 : (FILTER ? 512 : 1024) / kThreads;
-    static constexpr bool kTables = LOGM <= 13;           // the tables fit beside z
+    static constexpr bool kTables = LOGM <= 13;           // all tables fit beside z, at 16384 that of |H|
     // twiddles w_N^(i m), m = 1 .. 15, of every radix-16 pass: 15 (M/16 + M/256 + ...)
     static constexpr int kTwiddles = kPasses == 1 ? 0 : 15 * (T + (kPasses > 2 ? T / 16 : 0) + (kPasses > 3 ? T / 256 : 0));
-    static constexpr size_t kSmem = FILTER ? (size_t)kPairs * M * 8 + (kTables ? (size_t)M * 8 + kTwiddles * 8 : 0)
+    static constexpr size_t kSmem = FILTER ? (size_t)kPairs * M * 8 + (size_t)M * 4 + (kTables ? (size_t)M * 4 + kTwiddles * 8 : 0)
                                            : kTables ? (size_t)M * 4 : 0;
 };
 
 // Size of H at FFT bin k, as ktmApplyRhoFilter.m:33 pairs omega = 2 pi kk / Dr with the
 // shifted spectrum (kk = k - M for k >= M/2): 2D |w|; 2.5D sqrt|w| e^{i pi/4 sgn w}, both
 // parts of size sqrt(|w| / 2); 3D i w, zero at Nyquist.  |w| is the sum of two floats, and the
-// root of the larger one takes one Newton step against the sum: 6 million sizes (dt from 1e-5 to
-// 1 s, k to 8192) are the doubles of the formula rounded once, 4 % of the 2.5D ones are not if
+// approximate root takes one Newton step against both: 6 million sizes (dt from 1e-5 to 1 s, k to
+// 8192, roots 2^-22 off) are the doubles of the formula rounded once; 4 % of the 2.5D ones are not if
 // the root is taken of |w| already rounded.
 template <int M>
 __device__ __forceinline__ float rho_size(const PrepArgs& a, int k)
@@ -190,8 +190,9 @@ __device__ __forceinline__ float rho_size(const PrepArgs& a, int k)
     const int kk = k < (M >> 1) ? k : k - M;
     const float f = fabsf((float)kk), w = fmaf(f, a.wHi, f * a.wLo);
     if (a.rho == KTM_RHO_25D) {
-        const float hi = __fmul_rn(f, a.wHi), lo = fmaf(f, a.wHi, -hi) + f * a.wLo, s = __fsqrt_rn(hi);
-        return f > 0.0f ? fmaf(fmaf(-s, s, hi) + lo, 0.5f / s, s) : 0.0f;
+        const float hi = __fmul_rn(f, a.wHi), lo = fmaf(f, a.wLo, fmaf(f, a.wHi, -hi));
+        const float y = dev::rsqrt_approx(hi), s = hi * y;
+        return f > 0.0f ? fmaf(fmaf(-s, s, hi) + lo, 0.5f * y, s) : 0.0f;
     }
     return a.rho == KTM_RHO_3D && k == (M >> 1) ? 0.0f : w;
 }
@@ -211,7 +212,7 @@ __global__ void __launch_bounds__(FftShape<LOGM, FILTER>::kThreads, FftShape<LOG
     float2* zs = reinterpret_cast<float2*>(smem_raw) + (size_t)sub * M;
     // z of each pair, twiddles, |H| [E][T], fold weights [M]
     float2* twTab = reinterpret_cast<float2*>(smem_raw) + (FILTER ? S::kPairs * M : 0);
-    float* hTab = reinterpret_cast<float*>(twTab + (FILTER ? S::kTwiddles : 0));
+    float* hTab = reinterpret_cast<float*>(twTab + (FILTER && S::kTables ? S::kTwiddles : 0));
     float* wTab = hTab + (FILTER ? M : 0);
 
     // frequency of the last forward pass's output m of group g: the hexadecimal digits of
@@ -242,8 +243,8 @@ __global__ void __launch_bounds__(FftShape<LOGM, FILTER>::kThreads, FftShape<LOG
             v = cmul(v, conj_if(w, conj));
         }
     };
-    if (S::kTables) {
-        if (FILTER) {
+    if (FILTER || S::kTables) {
+        if (FILTER && S::kTables) {
             int o = 0;
 #pragma unroll
             for (int q = 0; q + 1 < P; q++) {
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__(FftShape<LOGM, FILTER>::kThreads, FftShape<LOG
         for (int v = threadIdx.x; v < M; v += S::kThreads) {
             const int u = v / T, g = v % T + T * (u / R);
             if (FILTER) hTab[v] = rho_size<M>(a, bin(g, u % R));
-            wTab[v] = (FILTER ? 1.0f / (float)M : 1.0f) * (a.prefold ? sqrtf((float)v * a.dt) : 1.0f);
+            if (S::kTables) wTab[v] = (FILTER ? 1.0f / (float)M : 1.0f) * (a.prefold ? sqrtf((float)v * a.dt) : 1.0f);
         }
         __syncthreads();
     }
@@ -319,7 +320,7 @@ __global__ void __launch_bounds__(FftShape<LOGM, FILTER>::kThreads, FftShape<LOG
                 for (int m = 0; m < R; m++) {
                     // bin m M / R + (bins of g): negative frequencies from m = R / 2 on, where bin
                     // M / 2 (Nyquist, g = 0) keeps the real part alone
-                    const float h = S::kTables ? hTab[(u * R + m) * T + t] : rho_size<M>(a, bin(g, m));
+                    const float h = hTab[(u * R + m) * T + t];
                     const float i = 2 * m < R ? im : 2 * m == R && g == 0 ? 0.0f : -im;
                     const float2 x = v[slot<R>(m)];
                     const float px = h * x.x, py = h * x.y;
