@@ -52,13 +52,6 @@ struct PrepArgs {
     float wHi, wLo;          // 2 pi / dt (pi / dt for the 2.5D filter) in two floats
 };
 
-// input sample n of the trace at p (IBM words converted as ktmIBM32toIEEE does)
-__device__ __forceinline__ float load_in(const float* p, int n, int ibm)
-{
-    if (ibm) return dev::ibm32_to_f32(reinterpret_cast<const uint32_t*>(p)[n]);
-    return p[n];
-}
-
 __device__ __forceinline__ void to_sample(float& d, float v) { d = v; }
 __device__ __forceinline__ void to_sample(__half& d, float v) { d = __float2half_rn(v); }
 __device__ __forceinline__ void to_sample(__nv_bfloat16& d, float v) { d = __float2bfloat16_rn(v); }
@@ -404,32 +397,69 @@ __global__ void __launch_bounds__(FftShape<LOGM, FILTER>::kThreads, FftShape<LOG
     }
 }
 
-// Traces longer than a transform, without a filter: one warp per trace reads it once for the
-// maximum (not for F32) and once more, from cache, to fold, scale and store it.
-constexpr int kPackWarps = 8;
+// Traces longer than a transform, without a filter: a CTA of 1024 threads per trace holds it in
+// registers between the maximum and the store, all its loads in flight at once.  1000 traces of
+// 20,000 samples to F16: 47 us (120 MB, 2.5 TB/s: one CTA an SM, its load, barrier and store in
+// turn), one trace 7; a warp per trace that reads it twice took 446 and 121, a CTA per pair in
+// shared memory 119 and 17.  From 8193 to 16384 samples the transform's kernel without its passes
+// is the faster (2441 traces of 8193: 49 us against 74): its CTAs stay for several pairs.
+constexpr int kPackThreads = 1024, kPackSamples = kMaxSmemBytes / 8;
 template <class OUT>
-__global__ void __launch_bounds__(kPackWarps * 32) pack_kernel(PrepArgs a)
+__global__ void __launch_bounds__(kPackThreads) pack_kernel(PrepArgs a)
 {
-    const int lane = threadIdx.x & 31;
-    const int k = blockIdx.x * kPackWarps + (threadIdx.x >> 5);
-    if (k >= a.ntr) return;
+    constexpr int E = (kPackSamples + kPackThreads - 1) / kPackThreads;
+    __shared__ float red[kPackThreads / 32];
+    const int t = threadIdx.x, k = blockIdx.x;
     const float* x = a.in + (size_t)k * a.inStride;
-    auto value = [&](int n) {
-        if (n <= 0 || n >= a.nt) return 0.0f;
-        const float v = load_in(x, n, a.ibm);
-        return a.prefold ? v * sqrtf((float)n * a.dt) : v;
-    };
+    float z[E];
+    if (a.ibm) {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(x);
+        bool other = false;
+#pragma unroll
+        for (int j = 0; j < E; j++) {
+            const int n = t + kPackThreads * j;
+            z[j] = dev::ibm32_usual(n < a.nt ? w[n] : 0u, other);
+        }
+        if (other) {
+#pragma unroll
+            for (int j = 0; j < E; j++) {
+                const int n = t + kPackThreads * j;
+                if (n < a.nt) z[j] = dev::ibm32_any(w[n]);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < E; j++) {
+            const int n = t + kPackThreads * j;
+            z[j] = n < a.nt ? x[n] : 0.0f;
+        }
+    }
+    if (t == 0) z[0] = 0.0f;
     float m = 0.0f;
+#pragma unroll
+    for (int j = 0; j < E; j++) {
+        const int n = t + kPackThreads * j;
+        if (a.prefold && n < a.nt) z[j] *= sqrtf((float)n * a.dt);
+        m = fmaxf(m, fabsf(z[j]));
+    }
     if (a.fmt != KTM_FMT_F32) {
-#pragma unroll 8
-        for (int n = lane; n < a.nt; n += 32) m = fmaxf(m, fabsf(value(n)));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if ((t & 31) == 0) red[t >> 5] = m;
+        __syncthreads();
+        m = red[t & 31];
+#pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     }
     const float s = trace_scale(a.fmt, m), inv = 1.0f / s;
     OUT* out = static_cast<OUT*>(a.out) + (size_t)out_slot(a, k) * a.pitch;
-#pragma unroll 8
-    for (int n = lane; n < a.pitch; n += 32) to_sample(out[n], value(n) * inv);
-    if (lane == 0) a.scale[out_slot(a, k)] = s;
+#pragma unroll
+    for (int j = 0; j < E; j++) {
+        const int n = t + kPackThreads * j;
+        if (n < a.pitch) to_sample(out[n], z[j] * inv);
+    }
+    for (int n = t + kPackThreads * E; n < a.pitch; n += kPackThreads) to_sample(out[n], 0.0f);
+    if (t == 0) a.scale[out_slot(a, k)] = s;
 }
 
 template <int LOGM, bool FILTER>
@@ -525,10 +555,10 @@ int prepare_traces(const ktm_prep* p)
     if ((size_t)a.nt * sizeof(float2) > (size_t)kMaxSmemBytes)
         return set_error(KTM_ERR_LIMIT, "prepare: tracePts > %d", kMaxSmemBytes / 8);
     if (a.nt > kMaxFft) {
-        const unsigned grid = (unsigned)((a.ntr + kPackWarps - 1) / kPackWarps);
-        if (a.fmt == KTM_FMT_F32) pack_kernel<float><<<grid, kPackWarps * 32, 0, s>>>(a);
-        else if (a.fmt == KTM_FMT_F16) pack_kernel<__half><<<grid, kPackWarps * 32, 0, s>>>(a);
-        else pack_kernel<__nv_bfloat16><<<grid, kPackWarps * 32, 0, s>>>(a);
+        const unsigned grid = (unsigned)a.ntr;
+        if (a.fmt == KTM_FMT_F32) pack_kernel<float><<<grid, kPackThreads, 0, s>>>(a);
+        else if (a.fmt == KTM_FMT_F16) pack_kernel<__half><<<grid, kPackThreads, 0, s>>>(a);
+        else pack_kernel<__nv_bfloat16><<<grid, kPackThreads, 0, s>>>(a);
         KTM_CUDA_TRY(cudaGetLastError());
         return KTM_OK;
     }

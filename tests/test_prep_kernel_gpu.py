@@ -154,3 +154,40 @@ def test_the_filter_is_rounded_once(cuda, ktm_lib, nt, opt):
             want = size * [0, c, c - s, -s][opt]
             want[0] = 0.0
         assert np.array_equal(got, np.float32(want)), (dt, got, want)
+
+
+@pytest.mark.parametrize("fmt", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("words,prefold", [(False, False), (False, True), (True, False)])
+@pytest.mark.parametrize("ntr,nt,extra", [(1, 8193, 0), (3, 16384, 8), (2, 17408, 0), (5, 17409, 16), (301, 16385, 0),
+                                          (2, 28673, 64), (3, 29056, 1024)])
+def test_long_traces_equal_the_plain_arithmetic(cuda, ktm_lib, ntr, nt, extra, words, prefold, fmt):
+    """A CTA per trace, around multiples of its threads, with guards past its registers."""
+    import torch
+
+    import ktm
+    from ktm import synth
+    rng = np.random.default_rng(nt)
+    x = (rng.standard_normal((ntr, nt + 3)) * 2.0 ** rng.integers(-9, 9, (ntr, 1))).astype(np.float32)
+    if words:
+        w = synth.encode_ibm32(x)
+        w[0, 5] = 0x7fffffff                            # 16^63: outside the FP32 range
+        src = torch.as_tensor(w.view(np.int32)).to(cuda)
+        flt = torch.empty((ntr, nt + 3), device=cuda)
+        ktm_lib.ktmIBM32toIEEEDevice(src.data_ptr(), flt.data_ptr(), src.numel(), None)
+        x = flt.cpu().numpy()
+    else:
+        src = torch.as_tensor(x).to(cuda)
+    dtype = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}[fmt]
+    out = torch.full((ntr, ktm.packed_pitch(nt, fmt) + extra), 7.0, device=cuda, dtype=dtype)
+    p = _prepare(src, 0.002, 0, prefold, fmt, nt=nt, out=out)
+    v = x[:, :nt].copy()
+    if prefold:
+        v *= np.sqrt(np.arange(nt, dtype=np.float32) * np.float32(0.002))
+    v[:, 0] = 0.0
+    top = np.abs(v).max(axis=1)
+    s = np.ones(ntr, np.float32) if fmt == "f32" else (top / np.float32(32768.0 if fmt == "f16" else 1.0))
+    with np.errstate(over="ignore", invalid="ignore"):
+        want = torch.as_tensor(v * (np.float32(1.0) / s)[:, None]).to(dtype)
+    assert np.array_equal(p.scale.cpu().numpy(), s)
+    assert torch.equal(torch.nan_to_num(p.data[:, :nt].cpu().float()), torch.nan_to_num(want.float()))
+    assert not p.data[:, nt:].any()
