@@ -564,7 +564,7 @@ int row_ctas(const Geometry& g, int wt, size_t* smem)
 template <int WT>
 int launch_rows(const RowArgs& ra, dim3 grid, size_t smem, cudaStream_t s)
 {
-    KTM_CUDA_TRY(cudaFuncSetAttribute(demigrate_row_kernel<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KTM_CUDA_TRY(allow_smem(demigrate_row_kernel<WT>, smem));
     demigrate_row_kernel<WT><<<grid, kRowWarps<WT> * 32, smem, s>>>(ra);
     KTM_CUDA_TRY(cudaGetLastError());
     return KTM_OK;
@@ -677,8 +677,7 @@ int launch_demigrate(const Geometry& g, const float* midX, const float* midY, co
     dim3 grid((unsigned)chunks, (unsigned)blocks);
 #define KTM_ADJ_LAUNCH(P, W)                                                                    \
     do {                                                                                        \
-        KTM_CUDA_TRY(cudaFuncSetAttribute(demigrate_merge_kernel<P, W>,                        \
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        KTM_CUDA_TRY(allow_smem(demigrate_merge_kernel<P, W>, smem));                           \
         demigrate_merge_kernel<P, W><<<grid, kAdjThreads, smem, s>>>(a);                       \
     } while (0)
     if (wt == 2 && pick != KTM_PICK_LINEAR)

@@ -587,7 +587,7 @@ int launch_block(const FastArgs& a, cudaStream_t stream, int smCount)
                                         "stage limit", a.pitch);
     const size_t smem = chunk_layout(st, SH::kWarps, a.pitch, esize, g.nt, kTable).total;
     auto kern = fast_kernel<SH, R, PICK, FMT, PRE, GRAD>;
-    KTM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KTM_CUDA_TRY(allow_smem(kern, smem, kMaxDynamic));
 
     const long long cols = (long long)g.nx * g.ny;
     const unsigned gx = (unsigned)((cols + SH::kWarps - 1) / SH::kWarps);
@@ -939,8 +939,7 @@ int launch_batch_t(const FastArgs* jobs, int njobs, cudaStream_t s)
         e = cudaGetLastError();
     }
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(batch_kernel<SH, R, PICK, FMT, PRE>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = allow_smem(batch_kernel<SH, R, PICK, FMT, PRE>, smem, kMaxDynamic);
     if (e == cudaSuccess) {
         const int grid = (int)std::min<size_t>((size_t)ctas, sorted.size());
         batch_kernel<SH, R, PICK, FMT, PRE><<<grid, SH::kThreads, smem, s>>>(dJobs, dChunks, dTiles,
@@ -1102,8 +1101,7 @@ int wait_selftest(int stall, unsigned long long limitNs, unsigned* checksum)
     int rc = KTM_OK;
     cudaError_t e = cudaMemsetAsync(src, 0x01, kBytes, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(out, 0, 64, s);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(wait_selftest_kernel,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+    if (e == cudaSuccess) e = allow_smem(wait_selftest_kernel, kBytes, kBytes);
     if (e == cudaSuccess) {
         wait_selftest_kernel<<<1, 256, kBytes, s>>>(src, kBytes, stall, limitNs, out);
         e = cudaGetLastError();

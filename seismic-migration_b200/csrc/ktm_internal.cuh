@@ -37,6 +37,17 @@ struct Geometry {
 // Largest dynamic shared memory a kernel here asks for (B200: 227 KB per CTA).
 constexpr int kMaxSmemBytes = 227 * 1024;
 
+// Lets `kern` have `smem` bytes of dynamic shared memory.  The limit is the kernel's, not the
+// launch's: it is always set to the same `most`, so that host threads whose calls differ in size
+// cannot lower it under one another between this and the launch.  Below the 48 KB that every
+// kernel may have nothing is set.
+template <class K>
+cudaError_t allow_smem(K kern, size_t smem, size_t most = kMaxSmemBytes)
+{
+    if (smem + 1024 <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 // Reference-mode kernel launch (ktm_ref.cu).  All pointers are device memory.
 int launch_reference(const Geometry& g, const float* midX, const float* midY,
                      const float* offX, const float* offY, const float* traces,

@@ -467,7 +467,7 @@ int launch_filter(const PrepArgs& a, cudaStream_t s)
 {
     using S = FftShape<LOGM, FILTER>;
     auto kern = prep_kernel<LOGM, FILTER>;
-    KTM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem));
+    KTM_CUDA_TRY(allow_smem(kern, S::kSmem, S::kSmem));
     int dev = 0, sm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);

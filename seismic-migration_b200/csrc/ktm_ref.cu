@@ -499,8 +499,7 @@ int launch_r(RefArgs a, const RefSplit& sp, cudaStream_t stream)
     a.chunk = ref_chunk(g, sp.warps, sp.perSm);
     const size_t smem = ref_smem(a.chunk, g.stride, g.nt, sp.warps).total;
     auto kern = reference_kernel<R>;
-    KTM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+    KTM_CUDA_TRY(allow_smem(kern, smem));
     const long long cols = (long long)g.nx * g.ny;
     const long long groups = (cols + sp.warps - 1) / sp.warps;
     const long long grid = groups * ((g.nz + 32LL * R - 1) / (32 * R));

@@ -89,8 +89,7 @@ extern "C" int ktmSynthesizeTraces(int traceNo, int tracePts, float sampleRate, 
     a.dt = (double)sampleRate; a.freq = freq; a.noise = noise; a.seed = seed;
     a.midX = midX; a.midY = midY; a.offX = offX; a.offY = offY; a.scat = scatterers; a.out = out;
     const size_t smem = (size_t)tracePts * sizeof(float);
-    KTM_CUDA_TRY(cudaFuncSetAttribute(ktm::synth_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+    KTM_CUDA_TRY(ktm::allow_smem(ktm::synth_kernel, smem));
     ktm::synth_kernel<<<traceNo, 256, smem, static_cast<cudaStream_t>(stream)>>>(a);
     KTM_CUDA_TRY(cudaGetLastError());
     return ktm::set_ok();
