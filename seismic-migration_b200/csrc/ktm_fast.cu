@@ -537,34 +537,33 @@ Stages fast_stages(const FastArgs& a, int esize, bool table)
 }
 
 // Partial images of a launch at most: an image of more than half of this is written in place.
-constexpr size_t kPartialBytes = 64u << 20;
+constexpr size_t kPartialBytes = 256u << 20;
 
-// Trace slices of a launch of `base` CTAs per slice on `slots` resident CTAs: the number with
-// the least estimated time in microseconds.  A CTA takes R / 16 for a trace, times the share of
-// the image that an aperture covers, and 2 + 6 R / 16 for its prologue, first copy and write-out.
-// Columns keep uneven numbers of traces, so that the longest CTA of a single round takes 1.3 of
-// the mean, two rounds 2.4, and more end half a round past it.  Partial images are written and
-// read once, and one more kernel (4) sums them.
-// Fitted to 112 launches (1 to 22,500 columns, 33 to 1501 samples, 100 to 60,000 traces), each
-// in 1 to 64 slices: the choice is on average 2 % off the best of them.  128 x 751 image, 6144
-// traces without aperture: 443 us in the 11 slices that fit at once, 354 in 64; 256 x 1001,
-// 1500 traces with an aperture of 700 m: 88 us in 6, 146 in 64.
+// Trace slices of a launch of `base` CTAs per slice on `slots` resident CTAs: the number
+// with the least estimated time, in traces of a CTA: a CTA takes its traces, times the share of the
+// image that an aperture covers, + 8 for its prologue, and the last ones end half a CTA past the
+// mean (columns keep uneven numbers of traces, and a line sorted by offset has slices without any:
+// 88 x 225 line, 4488 traces of 226 samples, 47 us in the 37 slices that fit at once, 34 in 64;
+// 1000 x 1001, 200 traces, aperture 700 m, 53 us without the share, 39 in one slice); plus the
+// partial images (a trace takes about 1 us at R = 16, 6.5 MB of partial images the same).
+// Estimates fitted to random surveys (prologue by R, whole rounds) gained 5 % there and lost up to
+// a quarter on sorted lines.
 int choose_slices(const FastArgs& a, long long base, int slots, int R)
 {
     const Geometry& g = a.g;
+    const int ntr = g.ntr;
     const size_t nimg = (size_t)g.nx * g.ny * g.nz;
-    const int most = (int)std::min<size_t>(std::max(1, std::min(64, g.ntr / 4)),
-                                           std::max<size_t>(1, kPartialBytes / (nimg * sizeof(float))));
     auto covered = [&](float extent) { return std::min(1.0f, 2.0f * a.aperture / std::max(fabsf(extent), 1e-30f)); };
     const float share = a.aperture > 0.0f ? std::max(0.1f, covered((float)g.nx * g.dx) * covered((float)g.ny * g.dy)) : 1.0f;
-    const float run = (float)R / 16.0f;
+    const int most = (int)std::min<size_t>(std::max(1, std::min(64, ntr / 8)),
+                                           std::max<size_t>(1, kPartialBytes / (nimg * sizeof(float))));
     int best = 1;
     float least = 3.0e38f;
     for (int s = 1; s <= most; s++) {
-        const float per = (float)((g.ntr + s - 1) / s) * run * share + 2.0f + 6.0f * run;
-        const float r = (float)(base * s) / (float)slots;
-        const float rounds = r <= 1.0f ? 1.3f : r <= 2.0f ? 2.4f : r + 0.5f;
-        const float cost = rounds * per + (s > 1 ? (float)s * (float)nimg * (8.0f / 6.5e6f) + 4.0f : 0.0f);
+        const float per = (float)((ntr + s - 1) / s) * share + 8.0f;
+        const float rounds = std::max(1.0f, (float)(base * s) / (float)slots) + 0.5f;
+        const float copies = s > 1 ? (float)s * (float)nimg * (8.0f / 6.5e6f) * 16.0f / (float)R : 0.0f;
+        const float cost = rounds * per + copies;
         if (cost < least) {
             least = cost;
             best = s;

@@ -1,5 +1,5 @@
-"""Trace slices of the fast migration: their partial images stay within 64 MiB whatever the
-image, and a call for which they do not fit into the device's memory runs without them."""
+"""Trace slices of the fast migration: their partial images stay within 256 MiB whatever
+the image, and a call for which they do not fit into the device's memory runs without them."""
 from __future__ import annotations
 
 import pytest
@@ -27,8 +27,8 @@ def _reserved():
     return memory_stats()["reserved"]
 
 
-@pytest.mark.parametrize("nx,ny,nz,ntr,nt", [(200, 100, 1501, 2500, 90), (60, 60, 1001, 4000, 300), (700, 1, 300, 50000, 60),
-                                             (100, 30, 2000, 30000, 40)])
+@pytest.mark.parametrize("nx,ny,nz,ntr,nt", [(200, 200, 1501, 2500, 90), (100, 150, 1501, 10000, 100), (700, 1, 300, 50000, 60),
+                                             (200, 100, 1000, 30000, 40)])
 def test_partial_images_are_bounded(cuda, ktm_lib, nx, ny, nz, ntr, nt):
     import torch
 
@@ -40,7 +40,7 @@ def test_partial_images_are_bounded(cuda, ktm_lib, nx, ny, nz, ntr, nt):
     job.run()
     torch.cuda.synchronize()
     # the pool maps its memory in pieces of 32 MiB
-    assert _reserved() - before <= 64 * MB + 32 * MB
+    assert _reserved() - before <= 256 * MB + 32 * MB
 
 
 def test_without_room_for_partial_images(cuda, ktm_lib):
@@ -48,7 +48,7 @@ def test_without_room_for_partial_images(cuda, ktm_lib):
     import torch
 
     from ktm._lib import check, memory_stats
-    job = _job(cuda, 60, 60, 1001, 4000, 300)
+    job = _job(cuda, 100, 100, 1001, 4000, 300)
     want = job.run().clone()
     torch.cuda.synchronize()
     assert memory_stats()["allocations"] > 0
@@ -61,7 +61,7 @@ def test_without_room_for_partial_images(cuda, ktm_lib):
                 taken.append(torch.empty(size, dtype=torch.uint8, device=cuda))
             except torch.cuda.OutOfMemoryError:
                 size //= 2
-        assert torch.cuda.mem_get_info()[0] < 14 * MB          # less than one partial image
+        assert torch.cuda.mem_get_info()[0] < 64 * MB          # less than two partial images
         job.run()
         torch.cuda.synchronize()
     finally:
