@@ -76,8 +76,8 @@ struct CtaShape {
     static constexpr size_t kBudget = (size_t)KB * 1024;
     static constexpr bool kFull = FULL != 0;
 };
-using Shape24 = CtaShape<24, 1, 220, 1>;
-using Shape12 = CtaShape<12, 2, 110, 0>;
+using Shape24 = CtaShape<24, 1, 226, 1>;
+using Shape12 = CtaShape<12, 2, 112, 0>;
 using Shape8 = CtaShape<8, 3, 74, 0>;
 template <class SH>
 constexpr bool shape_fits()
