@@ -207,18 +207,17 @@ __device__ __forceinline__ bool fast_tile(const FastArgs& a, Stages st, int colG
         S2[h] = pk(sv[0], sv[1]);
         acc[h] = pk(0.0f, 0.0f);
     }
+    // minima over the warp: no value is negative or NaN, so their bits order as they do
+    auto least = [](float v) { return __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(v))); };
 #pragma unroll
     for (int h = H - 1; h >= 0; h--) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            step[h].x = fminf(step[h].x, __shfl_xor_sync(0xffffffffu, step[h].x, o));
-            step[h].y = fminf(step[h].y, __shfl_xor_sync(0xffffffffu, step[h].y, o));
-        }
         if (h + 1 < H) step[h] = make_float2(fminf(step[h].x, step[h + 1].x), fminf(step[h].y, step[h + 1].y));
-        if (lane == 0) steps[h] = step[h];
+        if (kStepwise || h == 0) {
+            step[h] = make_float2(least(step[h].x), least(step[h].y));
+            if (lane == 0) steps[h] = step[h];
+        }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) nvalid += __shfl_xor_sync(0xffffffffu, nvalid, o);
+    nvalid = (int)__reduce_add_sync(0xffffffffu, (unsigned)nvalid);
     const float colX = g.x0 + (float)ci * g.dx, colY = g.y0 + (float)cj * g.dy;
     if (PRE == kWtTable) {
         for (int j = threadIdx.x; j <= g.nt; j += SH::kThreads) {
