@@ -512,13 +512,15 @@ __global__ void reduce_slices(float* __restrict__ out, const float* __restrict__
 // Traces per row buffer and buffers: as many traces as the shape's shared-memory budget
 // holds (at most kMaxChunk per buffer, or fewer when the caller caps them: chunkCap > 0),
 // in three buffers where each still gets 16 traces, else in two: the third lets the warps
-// drift further apart, fewer traces per buffer cost more of the per-chunk geometry.  chunk 0
+// drift further apart, fewer traces per buffer cost more of the per-chunk geometry.  No more than
+// the launch's traces need, which leaves the L1 cache its room (60 million samples, 8 F32 traces:
+// 318 us, 391 with all buffers).  chunk 0
 // for traces beyond the limit: two of them, with the weight table, exceed the largest
 // allocation a CTA can have.
 template <class SH>
 Stages fast_stages(const FastArgs& a, int esize, bool table)
 {
-    const int cap = a.chunkCap > 0 ? std::min(kMaxChunk, a.chunkCap) : kMaxChunk;
+    const int cap = std::min(a.chunkCap > 0 ? std::min(kMaxChunk, a.chunkCap) : kMaxChunk, std::max(1, a.g.ntr));
     auto fit = [&](int stages) {
         Stages s = {cap, stages};
         while (s.chunk > 1 && chunk_layout(s, SH::kWarps, a.pitch, esize, a.g.nt, table).total > SH::kBudget)
@@ -530,6 +532,7 @@ Stages fast_stages(const FastArgs& a, int esize, bool table)
         return Stages{0, 0};
     Stages s = fit(3);
     if (s.chunk < std::min(cap, 16)) s = fit(2);
+    s.stages = std::max(1, std::min(s.stages, (a.g.ntr + s.chunk - 1) / s.chunk));     // no buffer without a copy
     // the longest traces: two buffers leave no room for the warps' tables
     if (chunk_layout(s, SH::kWarps, a.pitch, esize, a.g.nt, table).total > kMaxDynamic) s.stages = 1;
     return s;
