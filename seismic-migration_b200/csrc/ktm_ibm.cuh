@@ -28,7 +28,7 @@ __device__ __forceinline__ float pow2_exact(int e)
 }
 
 // every word, the infinite powers and the 0 * inf case among them
-static __device__ __noinline__ float ibm32_any(uint32_t w)
+__device__ __forceinline__ float ibm32_to_f32(uint32_t w)
 {
     const float sign = (w & 0x80000000u) ? -1.0f : 1.0f;
     const float q = __fdiv_rn(__uint2float_rn(w & 0x00ffffffu), 16777215.0f);
@@ -40,10 +40,13 @@ static __device__ __noinline__ float ibm32_any(uint32_t w)
     return __fmul_rn(__fmul_rn(sign, q), p);
 }
 
+// the same out of line, for the rare words of kernels that convert the usual ones below
+static __device__ __noinline__ float ibm32_any(uint32_t w) { return ibm32_to_f32(w); }
+
 // Words whose power of two is a normal number (exponents 33 to 95), and zeros with smaller
 // ones: one multiply for the quotient, one residual step (for all 2^24 fractions it gives
 // the correctly rounded quotient) and the power from its bits, about 12 instructions and no
-// branch.  Sets `other` for a word that ibm32_any has to convert.  All 2^32 words give the
+// branch: for kernels that are bound by issue.  Sets `other` for a word that ibm32_any has to convert.  All 2^32 words give the
 // same bits by the two together as by ibm32_any alone (checked on the GPU).  4097 traces of
 // 1001 words through the 2.5D filter: 17 us, with the division and its selects per word 29.
 __device__ __forceinline__ float ibm32_usual(uint32_t w, bool& other)
@@ -56,12 +59,5 @@ __device__ __forceinline__ float ibm32_usual(uint32_t w, bool& other)
     // 2^(4 (E - 64)) with the word's sign: (4 E - 256 + 127) << 23
     return __fmul_rn(q, __uint_as_float(((max(e, 0x21000000u) << 1) - (129u << 23)) | (w & 0x80000000u)));
 }
-__device__ __forceinline__ float ibm32_to_f32(uint32_t w)
-{
-    bool other = false;
-    const float v = ibm32_usual(w, other);
-    return other ? ibm32_any(w) : v;
-}
-
 }  // namespace dev
 }  // namespace ktm
