@@ -311,8 +311,10 @@ int migrate_impl(const ktm_job* j)
     // host buffers: copy in, run, copy out, synchronise
     const size_t ntr = (size_t)g.ntr, nimg = (size_t)g.nx * g.ny * g.nz;
     const size_t nvel = j->velocityCube ? nimg : (size_t)g.nz;
-    // a small image comes back together with the count of waits that ran out
-    const bool small = nimg > 0 && nimg * 4 <= Staged::kTogether * 4;
+    // a small image comes back together with the count of waits that ran out; a larger one is worth
+    // its own copy, straight into a pinned buffer (260 x 251 image, 512 pinned traces: 124 us, 149
+    // through a buffer of this call)
+    const bool small = nimg > 0 && nimg * 4 <= Staged::kTogether;
     unsigned stalls = 0;
     {
         Staged st(s);
