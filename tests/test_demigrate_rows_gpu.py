@@ -95,3 +95,12 @@ def test_accumulates(cuda, ktm_lib, ntr):
     plain = _run(cuda, c, False)
     start = np.random.default_rng(1).standard_normal(plain.shape).astype(np.float32)
     _same(_run(cuda, c, False, start=start.copy()), start + plain)
+
+
+@pytest.mark.parametrize("weight", ["prefold", "table"])
+@pytest.mark.parametrize("nx,ntr,nz,dz", [(40, 11, 300, 0.002), (40, 12, 300, 0.002), (257, 127, 70, 0.002), (257, 128, 70, 0.002), (257, 511, 70, 0.002), (257, 512, 70, 0.002),
+                                          (30, 40, 63, 0.004), (30, 40, 64, 0.004), (30, 40, 63, 0.002)])
+def test_either_side_of_the_rules(cuda, ktm_lib, nx, ntr, nz, dz, weight):
+    """Few traces, shallow images: whichever kernel takes the call, the sums are the same."""
+    c = _case(nx + ntr, nx, ntr, 300, nz, dz)
+    _same(_run(cuda, c, False, weight=weight), _run(cuda, c, True, weight=weight))

@@ -17,7 +17,7 @@ def test_without_room_for_the_model_copy(cuda, ktm_lib, graph):
     from ktm import inverse
     from ktm._lib import check
     # a shallow image: the copy pads its 33 samples to 256 (25 MiB -> 195 MiB)
-    nx, nz, ntr, nt = 200000, 33, 64, 200
+    nx, nz, ntr, nt = 200000, 33, 160, 200
     g = torch.Generator(device=cuda)
     g.manual_seed(1)
     c = [torch.rand(ntr, device=cuda, generator=g) * 0.5 * nx for _ in range(2)]
