@@ -642,6 +642,13 @@ int launch_demigrate(const Geometry& g, const float* midX, const float* midY, co
     int dev = 0, sm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
+    const int wt = weightMethod == KTM_WEIGHT_SQRT ? 1 : weightMethod == KTM_WEIGHT_PREFOLD ? 2 : 0;
+    // the shared rows' limit is every call's: the kernel with a row per warp may not find its memory.
+    // The sqrt(j dt) table only for the table weight; the coordinates' alignment pad
+    const size_t fixed = (wt == 0 ? (size_t)padded_pitch(g.nt + 1) * sizeof(float2) : 0) + 64;
+    const size_t perTrace = (size_t)padded_pitch(pitch) * sizeof(float) + 4 * sizeof(float);
+    if (!empty && fixed + perTrace > (size_t)kMaxSmemBytes)
+        return set_error(KTM_ERR_LIMIT, "demigrate: tracePts=%d exceeds the shared-memory limit", g.nt);
     const size_t need = empty ? 0 : demigrate_scratch(g, velCube, pick, weightMethod);
     void* own = nullptr;
     if (need && !scratch && mayAllocate && pool_malloc(&own, need, s) != cudaSuccess) {
@@ -657,14 +664,8 @@ int launch_demigrate(const Geometry& g, const float* midX, const float* midY, co
     if (!accumulate && g.ntr > 0)
         KTM_CUDA_TRY(cudaMemsetAsync(data, 0, pitchBytes * g.ntr, s));
     if (empty) return KTM_OK;
-    const int wt = weightMethod == KTM_WEIGHT_SQRT ? 1 : weightMethod == KTM_WEIGHT_PREFOLD ? 2 : 0;
-    // the sqrt(j dt) table only for the table weight; the coordinates' alignment pad
-    const size_t fixed = (wt == 0 ? (size_t)padded_pitch(g.nt + 1) * sizeof(float2) : 0) + 64;
-    const size_t perTrace = (size_t)padded_pitch(pitch) * sizeof(float) + 4 * sizeof(float);
     int chunk = 32;                     // at most 32: lane c evaluates trace c's geometry
     while (chunk > 1 && fixed + chunk * perTrace > kAdjSmemBudget) chunk--;
-    if (fixed + chunk * perTrace > (size_t)kMaxSmemBytes)
-        return set_error(KTM_ERR_LIMIT, "demigrate: tracePts=%d exceeds the shared-memory limit", g.nt);
     const size_t smem = fixed + chunk * perTrace;
 
     const int ncols = g.nx * g.ny;

@@ -104,3 +104,21 @@ def test_either_side_of_the_rules(cuda, ktm_lib, nx, ntr, nz, dz, weight):
     """Few traces, shallow images: whichever kernel takes the call, the sums are the same."""
     c = _case(nx + ntr, nx, ntr, 300, nz, dz)
     _same(_run(cuda, c, False, weight=weight), _run(cuda, c, True, weight=weight))
+
+
+def test_the_limit_is_every_calls(cuda, ktm_lib):
+    """Rows longer than shared memory are refused whatever kernel would take the call."""
+    import torch
+
+    import ktm
+    from ktm._lib import lib
+    c = _case(3, 20, 40, 300, 100, 0.002)
+    gx, gz, nt, mx, my, ox, oy, vel, img, ap = c
+    t = [torch.as_tensor(a).to(cuda) for a in (mx, my, ox, oy, vel, img)]
+    for pitch, ok in ((46000, True), (47000, False)):
+        data = torch.zeros((40, pitch), device=cuda)
+        job = ktm.Job(imageX=gx, imageY=(1, 1.0, 0.0), imageZ=gz, dt=0.004, midX=t[0], midY=t[1], offX=t[2], offY=t[3],
+                      velocity=t[4], traces=ktm.PackedTraces(data, torch.ones(40, device=cuda), nt, "f32", False, 0),
+                      image=t[5], weight="prefold")
+        rc = lib().ktmDemigrate(C.byref(job.job), data.data_ptr(), pitch)
+        assert rc == (0 if ok else ktm._lib.KTM_ERR_LIMIT)
