@@ -295,8 +295,9 @@ demigrate_merge_kernel(AdjArgs a)
 // reductions.
 // 512 x 1001 image, 32,768 traces of 1001 samples, prefolded / table / sqrt weight:
 // 11.4 / 18.0 / 12.5 ms, against 14.7 / 18.5 / 15.4 with rows shared by the CTA; 100 columns,
-// 2000 traces 0.33 / 0.47 against 0.54 / 0.59.  Bound by issue (35 instructions a pair, three
-// quarters of the slots) and by the shared-memory pipe.
+// 2000 traces 0.32 / 0.44 against 0.56 / 0.60.  Bound by issue (35 instructions a pair, three
+// quarters of the slots) and by the shared-memory pipe.  At 64 registers it spills (36 / 60 / 20
+// bytes stored, 92 / 124 / 76 loaded).
 constexpr int kRowR = 8;
 constexpr int kRowRun = 32 * kRowR;
 // Warps per CTA, up to 32 warps per SM: small CTAs end at their own pace (512 x 1001 image,

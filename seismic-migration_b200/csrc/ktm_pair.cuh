@@ -161,8 +161,8 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n"); }
 
 // ---- bulk (TMA) copies global -> shared, completed on an mbarrier ----------
-// One thread initialises, arms and waits on the barrier; a __syncthreads after
-// its wait publishes the landed bytes to the rest of the CTA.
+// One thread initialises and arms the barrier; every warp that reads the landed bytes waits
+// on it itself, or one thread waits and a __syncthreads publishes them to the CTA.
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned arrivals)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(arrivals) : "memory");

@@ -20,8 +20,8 @@
 // n ^ ((n >> 4) & 15), which gives 16 neighbouring lanes 16 different 8-byte banks at
 // every pass's stride.  CTAs stay for several pairs and keep tables of the
 // twiddles (sincospif each), the filter and the fold weights in shared memory.
-// What bounds it: issue and the FP32 pipe, about 1700 instructions a thread and pair, three
-// quarters of the issue slots busy at 16 warps per SM.  62,500 traces of 1501 samples, 3D
+// What bounds it: issue and the FP32 pipe, about 1700 instructions a thread and pair, 62 % of
+// the issue slots busy at 16 warps per SM.  62,500 traces of 1501 samples, 3D
 // filter to FP16: 297 us, where the radix-2 transform in shared memory (22 passes with a
 // barrier each, double-precision filter) took 2581; 4 bytes read and 2 written per sample
 // would take 86.  Without a filter the same kernel keeps the samples in registers between

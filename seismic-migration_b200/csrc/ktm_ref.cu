@@ -10,7 +10,8 @@
 //   * each image sample is owned by one lane, which adds the traces in increasing
 //     k, the order of the reference's outer loop (:56-59).
 //
-// Correct rounding without the library sequences (ref_pack): two traces go through
+// Correct rounding without the library sequences (ref_packs; the enumerations below were made once,
+// the tests compare whole migrations bit for bit): two traces go through
 // each packed f32x2 instruction, and inside the operand ranges below no special case
 // is left to test for.
 //   sqrt(a): y = rsqrt.approx(a), g = a y, s = g + (a - g^2) (y / 2), the residual and
