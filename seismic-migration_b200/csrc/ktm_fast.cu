@@ -549,7 +549,7 @@ constexpr size_t kPartialBytes = 256u << 20;
 // 1000 x 1001, 200 traces, aperture 700 m, 53 us without the share, 39 in one slice); plus the
 // partial images (a trace takes about 1 us at R = 16, 6.5 MB of partial images the same).
 // Estimates fitted to random surveys (prologue by R, whole rounds) gained 5 % there and lost up to
-// a quarter on sorted lines.
+// 40 % on sorted lines.
 int choose_slices(const FastArgs& a, long long base, int slots, int R)
 {
     const Geometry& g = a.g;
@@ -860,8 +860,8 @@ __global__ void __launch_bounds__(256) zero_images(const FastArgs* __restrict__ 
     }
 }
 
-// CTAs per image: one per 4096 samples of the largest, at most eight per SM over all images.  One job
-// of 60 million samples: 50 us, with 16 CTAs an image whatever its size 430.
+// CTAs per image: one per 4096 samples of the largest, at most eight per SM over all images.  A call of
+// one job, 60 million samples and 8 BF16 traces: 317 us, 632 with 16 CTAs an image whatever its size.
 int zero_ctas(const FastArgs* jobs, int njobs, int sm)
 {
     size_t most = 1;
