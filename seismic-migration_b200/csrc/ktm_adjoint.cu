@@ -553,11 +553,9 @@ __global__ void __launch_bounds__(kRowWarps<WT> * 32, 32 / kRowWarps<WT>) demigr
 // ms against 15.4).
 // A few traces give too few warps at one a trace, each with a block of columns to go through in turn,
 // where the shared rows bring 32 to a chunk of up to 32 traces: one trace into 100 columns 57 us
-// against 28, 12 traces 64 against 84; 24 into 2500 columns, most of them out of reach, 117 against
-// 58, 64 into 512 111 against 111 (with the weight table, which every CTA builds, 256 into 2500 296
-// against 203).  Images of a few samples with coarse steps or the weight table:
-// 300 columns of 33 samples, 20,000 traces 1.77 ms against 1.53, 2000 traces with the table 325 us
-// against 263.
+// against 28, 8 traces 117 against 73, 12 traces 64 against 84; 24 into 2500 columns, most of them
+// out of reach, 117 against 58, 64 into 512 111 against 111, 500 into 50 x 50 columns within reach
+// 1.03 ms against 2.02 (table weight).
 int row_ctas(const Geometry& g, int wt, size_t* smem)
 {
     const int nruns = (g.nz + kRowRun - 1) / kRowRun, warps = wt == 0 ? kRowWarps<0> : kRowWarps<1>;
@@ -565,8 +563,8 @@ int row_ctas(const Geometry& g, int wt, size_t* smem)
             (wt == 0 ? (size_t)padded_pitch(g.nt + 1) * sizeof(float2) : 0);
     const int ctas = (int)std::min<size_t>(32 / warps, (size_t)(227 * 1024) / (*smem + 1024));
     const bool coarse = !(2.0f * fabsf(g.dz) <= 1.05f * g.dt);
-    if (g.nt > 8192 || (wt == 0 && coarse) || (g.nz < 64 && (wt == 0 || coarse))) return 0;
-    if (g.ntr < ((long long)g.nx * g.ny <= 256 ? 12 : wt == 0 ? 512 : 128)) return 0;
+    if (g.nt > 8192 || (wt == 0 && coarse)) return 0;
+    if (g.ntr < ((long long)g.nx * g.ny <= 256 ? 10 : 64)) return 0;
     return ctas * warps >= (wt == 0 || coarse ? 32 : 16) ? ctas : 0;
 }
 
